@@ -32,39 +32,15 @@ GL_HD u64 gl_mulhi(u64 a, u64 b) {
 #endif
 }
 
-// (hi * 2^64 + lo) mod p with 2^64 = 2^32 - 1 and 2^96 = -1.
-GL_HD u64 gl_reduce(u64 lo, u64 hi) {
-  u64 hh = hi >> 32, hl = hi & GL_EPS;
-  u64 t0 = lo - hh;
-  if (lo < hh) t0 -= GL_EPS;
-  u64 t1 = (hl << 32) - hl;
-  u64 t2 = t0 + t1;
-  if (t2 < t1) t2 += GL_EPS;
-  return t2 >= GL_P ? t2 - GL_P : t2;
-}
 #ifdef __CUDA_ARCH__
-// Device versions on 32-bit carry chains.  Operands and results are canonical.
+// Device versions on 32-bit carry chains.  Operands and results are canonical.  On sm_100 an
+// instruction that takes or gives a carry issues at half the rate of a plain 32-bit add, and a
+// 32 x 32 -> 64-bit multiply(-add) at a quarter, so each of these forms is the one that measured
+// fastest among several with the same value: per SM and clock 10.6 gl_add, 15.9 gl_sub, 3.5
+// gl_mul and 0.98 ef_mul (8.8, 15.9, 2.6 and 0.76 with conditional corrections by wide
+// multiply-adds).
 __device__ __forceinline__ u64 gl_pack(uint32_t lo, uint32_t hi) {
   return ((u64)hi << 32) | lo;
-}
-// a + b: s = a + b (carry c1), and c2 = the carry of s + eps (that is, s >= p); exactly one of
-// them set means the canonical result is s + eps = s - p (mod 2^64) (a, b < p, so never both).
-// The correction s + (c1 + c2) eps is one wide multiply-add, which runs on the FMA pipe instead
-// of selects on the integer ALU pipe.
-__device__ __forceinline__ u64 gl_add(u64 a, u64 b) {
-  u64 r;
-  asm("{\n\t.reg .u32 s0, s1, d, c;\n\t.reg .u64 s;\n\t"
-      "add.cc.u32 s0, %1, %3;\n\t"
-      "addc.cc.u32 s1, %2, %4;\n\t"
-      "addc.u32 c, 0, 0;\n\t"
-      "add.cc.u32 d, s0, 0xffffffff;\n\t"
-      "addc.cc.u32 d, s1, 0;\n\t"
-      "addc.u32 c, c, 0;\n\t"
-      "mov.b64 s, {s0, s1};\n\t"
-      "mad.wide.u32 %0, c, 0xffffffff, s;\n\t}"
-      : "=l"(r)
-      : "r"((uint32_t)a), "r"((uint32_t)(a >> 32)), "r"((uint32_t)b), "r"((uint32_t)(b >> 32)));
-  return r;
 }
 // a - b: on a borrow, d = a - b + 2^64 and the result is d - eps = a - b + p.
 __device__ __forceinline__ u64 gl_sub(u64 a, u64 b) {
@@ -79,33 +55,48 @@ __device__ __forceinline__ u64 gl_sub(u64 a, u64 b) {
       : "r"((uint32_t)a), "r"((uint32_t)(a >> 32)), "r"((uint32_t)b), "r"((uint32_t)(b >> 32)));
   return gl_pack(d0, d1);
 }
-// (r0 + r1 2^32 + r2 2^64 + r3 2^96) mod p = (r0 + r1 2^32) - r3 + r2 (2^32 - 1).
-// u = lo - r3 (minus eps on a borrow), w = u + r2 eps (plus eps on a carry, which cannot carry
-// again), then the canonical w - p if w >= p.  The products and both conditional corrections
-// are wide multiplies/multiply-adds (FMA pipe).
+// a + b = a - (p - b): p - b lies in [1, p] and a < p, so gl_sub's single correction suffices.
+__device__ __forceinline__ u64 gl_add(u64 a, u64 b) { return gl_sub(a, GL_P - b); }
+// The canonical form of any 64-bit value: x >= p exactly when the high word is all ones and the
+// low word is not zero, and x - p is then (low - 1, 0).
+__device__ __forceinline__ u64 gl_canon_words(uint32_t lo, uint32_t hi) {
+  asm("{\n\t.reg .pred p, q;\n\t"
+      "setp.eq.u32 p, %1, 0xffffffff;\n\t"
+      "setp.ne.and.u32 q, %0, 0, p;\n\t"
+      "@q sub.u32 %0, %0, 1;\n\t"
+      "@q mov.u32 %1, 0;\n\t}"
+      : "+r"(lo), "+r"(hi));
+  return gl_pack(lo, hi);
+}
+// (r0 + r1 2^32 + r2 2^64 + r3 2^96 + r4 2^128) mod p for r4 < 2^31, with 2^64 = 2^32 - 1,
+// 2^96 = -1 and 2^128 = -2^32: V = lo - r4 2^32 - r3 - r2 + r2 2^32 lies in (-2^63 - 2^33, 2^65 -
+// 2^33), so V = v + k 2^64 with one k in {-1, 0, 1}, and v + k (2^32 - 1) cannot wrap again.
+__device__ __forceinline__ u64 gl_reduce5(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3,
+                                          uint32_t r4) {
+  uint32_t v0, v1;
+  asm("{\n\t.reg .u32 k, m;\n\t.reg .u64 w;\n\t"
+      "sub.cc.u32 %0, %2, %5;\n\t"
+      "subc.cc.u32 %1, %3, %6;\n\t"
+      "subc.u32 k, 0, 0;\n\t"
+      "sub.cc.u32 %0, %0, %4;\n\t"
+      "subc.cc.u32 %1, %1, 0;\n\t"
+      "subc.u32 k, k, 0;\n\t"
+      "add.cc.u32 %1, %1, %4;\n\t"
+      "addc.u32 k, k, 0;\n\t"
+      "neg.s32 m, k;\n\t"
+      "mov.b64 w, {%0, %1};\n\t"
+      "mad.wide.s32 w, m, 1, w;\n\t"
+      "mov.b64 {%0, %1}, w;\n\t"
+      "add.u32 %1, %1, k;\n\t}"
+      : "=&r"(v0), "=&r"(v1)
+      : "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(r4));
+  return gl_canon_words(v0, v1);
+}
 __device__ __forceinline__ u64 gl_reduce4(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-  u64 r;
-  asm("{\n\t.reg .u32 u0, u1, m, v0, v1, w0, w1, d, c;\n\t.reg .u64 v, w;\n\t"
-      "sub.cc.u32 u0, %1, %4;\n\t"
-      "subc.cc.u32 u1, %2, 0;\n\t"
-      "subc.u32 m, 0, 0;\n\t"
-      "sub.cc.u32 u0, u0, m;\n\t"
-      "subc.u32 u1, u1, 0;\n\t"
-      "mul.wide.u32 v, %3, 0xffffffff;\n\t"
-      "mov.b64 {v0, v1}, v;\n\t"
-      "add.cc.u32 w0, u0, v0;\n\t"
-      "addc.cc.u32 w1, u1, v1;\n\t"
-      "addc.u32 c, 0, 0;\n\t"
-      "mov.b64 w, {w0, w1};\n\t"
-      "mad.wide.u32 w, c, 0xffffffff, w;\n\t"
-      "mov.b64 {w0, w1}, w;\n\t"
-      "add.cc.u32 d, w0, 0xffffffff;\n\t"
-      "addc.cc.u32 d, w1, 0;\n\t"
-      "addc.u32 c, 0, 0;\n\t"
-      "mad.wide.u32 %0, c, 0xffffffff, w;\n\t}"
-      : "=l"(r)
-      : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
-  return r;
+  return gl_reduce5(r0, r1, r2, r3, 0);
+}
+__device__ __forceinline__ u64 gl_reduce(u64 lo, u64 hi) {
+  return gl_reduce4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
 }
 __device__ __forceinline__ u64 gl_mul(u64 a, u64 b) {
   const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32);
@@ -125,6 +116,16 @@ __device__ __forceinline__ u64 gl_mul(u64 a, u64 b) {
   return gl_reduce4(r0, r1, r2, r3);
 }
 #else
+// (hi * 2^64 + lo) mod p with 2^64 = 2^32 - 1 and 2^96 = -1.
+GL_HD u64 gl_reduce(u64 lo, u64 hi) {
+  u64 hh = hi >> 32, hl = hi & GL_EPS;
+  u64 t0 = lo - hh;
+  if (lo < hh) t0 -= GL_EPS;
+  u64 t1 = (hl << 32) - hl;
+  u64 t2 = t0 + t1;
+  if (t2 < t1) t2 += GL_EPS;
+  return t2 >= GL_P ? t2 - GL_P : t2;
+}
 GL_HD u64 gl_add(u64 a, u64 b) {
   u64 s = a + b;
   if (s < a) s += GL_EPS;
@@ -136,7 +137,7 @@ GL_HD u64 gl_mul(u64 a, u64 b) { return gl_reduce(a * b, gl_mulhi(a, b)); }
 GL_HD u64 gl_neg(u64 a) { return a ? GL_P - a : 0; }
 #ifdef __CUDACC__
 // Unreduced multiply-accumulate: acc (five 32-bit words, < 2^160) += a * b as a 128-bit product.
-// Sums of up to 2^32 products are exact; gl_acc_reduce brings the sum back into the field.
+// Sums of up to 2^31 products are exact; gl_acc_reduce brings the sum back into the field.
 struct Acc160 {
   uint32_t w[5];
 };
@@ -166,10 +167,10 @@ __device__ __forceinline__ void gl_mac(Acc160& acc, u64 a, u64 b) {
       : "r"(a0), "r"(a1), "r"(b0), "r"(b1));
 #endif
 }
-// (w0 + w1 2^32 + w2 2^64 + w3 2^96 + w4 2^128) mod p, with 2^128 = -2^32 mod p.
+// (w0 + w1 2^32 + w2 2^64 + w3 2^96 + w4 2^128) mod p.
 __device__ __forceinline__ u64 gl_acc_reduce(const Acc160& a) {
 #ifdef __CUDA_ARCH__
-  return gl_sub(gl_reduce4(a.w[0], a.w[1], a.w[2], a.w[3]), (u64)a.w[4] << 32);
+  return gl_reduce5(a.w[0], a.w[1], a.w[2], a.w[3], a.w[4]);
 #else
   return 0;
 #endif
