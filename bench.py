@@ -523,11 +523,11 @@ def rs_alu_floor(lib, ctx, log_m: int, log_n: int, measured_ms: float) -> dict:
     L._lib.check(lib.lgs_rs_alu_rates(ctx.handle, 4096, C.byref(r8), C.byref(mul)))
     N = 2 << log_n
     n2 = N >> 12
-    # pass A: four radix-8 stages (the first on a half-zero input, 8 of its 12 butterflies),
-    # 7 + 8 + 7 twiddle products per 8 values; pass B: log8(N2) stages, 15 products per 8
-    # values when N2 = 64 (one per value otherwise)
+    # pass A: four radix-8 stages (the first on a half-zero input, 8 of its 12 butterflies) and one
+    # table product per value; pass B: log8(N2) stages and one product per value.  The twiddles of
+    # order 64 between radix-8 digits are shifts in the packing, not products.
     r8_per = (2.0 / 3.0 + 3.0) / 8.0 + (math.log2(n2) / 3.0) / 8.0
-    mul_per = 22.0 / 8.0 + (15.0 / 8.0 if n2 == 64 else 1.0)
+    mul_per = 1.0 + (1.0 if n2 >= 4 else 0.0)
     values = float(1 << log_m) * N
     floor_ms = values * (r8_per / r8.value + mul_per / mul.value) * 1e3
     return {"floor_ms": round(floor_ms, 4), "frac_of_floor": round(floor_ms / measured_ms, 4),

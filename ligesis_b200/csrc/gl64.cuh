@@ -32,6 +32,8 @@ GL_HD u64 gl_mulhi(u64 a, u64 b) {
 #endif
 }
 
+GL_HD u64 gl_pack(uint32_t lo, uint32_t hi) { return ((u64)hi << 32) | lo; }
+
 #ifdef __CUDA_ARCH__
 // Device versions on 32-bit carry chains.  Operands and results are canonical.  On sm_100 an
 // instruction that takes or gives a carry issues at half the rate of a plain 32-bit add, and a
@@ -39,9 +41,6 @@ GL_HD u64 gl_mulhi(u64 a, u64 b) {
 // fastest among several with the same value: per SM and clock 10.6 gl_add, 15.9 gl_sub, 3.5
 // gl_mul and 0.98 ef_mul (8.8, 15.9, 2.6 and 0.76 with conditional corrections by wide
 // multiply-adds).
-__device__ __forceinline__ u64 gl_pack(uint32_t lo, uint32_t hi) {
-  return ((u64)hi << 32) | lo;
-}
 // a - b: on a borrow, d = a - b + 2^64 and the result is d - eps = a - b + p.
 __device__ __forceinline__ u64 gl_sub(u64 a, u64 b) {
   uint32_t d0, d1;
@@ -71,8 +70,9 @@ __device__ __forceinline__ u64 gl_canon_words(uint32_t lo, uint32_t hi) {
 // (r0 + r1 2^32 + r2 2^64 + r3 2^96 + r4 2^128) mod p for r4 < 2^31, with 2^64 = 2^32 - 1,
 // 2^96 = -1 and 2^128 = -2^32: V = lo - r4 2^32 - r3 - r2 + r2 2^32 lies in (-2^63 - 2^33, 2^65 -
 // 2^33), so V = v + k 2^64 with one k in {-1, 0, 1}, and v + k (2^32 - 1) cannot wrap again.
-__device__ __forceinline__ u64 gl_reduce5(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3,
-                                          uint32_t r4) {
+// gl_reduce_lazy leaves any representative below 2^64; gl_reduce5 the canonical one.
+__device__ __forceinline__ u64 gl_reduce_lazy(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3,
+                                              uint32_t r4) {
   uint32_t v0, v1;
   asm("{\n\t.reg .u32 k, m;\n\t.reg .u64 w;\n\t"
       "sub.cc.u32 %0, %2, %5;\n\t"
@@ -90,7 +90,12 @@ __device__ __forceinline__ u64 gl_reduce5(uint32_t r0, uint32_t r1, uint32_t r2,
       "add.u32 %1, %1, k;\n\t}"
       : "=&r"(v0), "=&r"(v1)
       : "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(r4));
-  return gl_canon_words(v0, v1);
+  return gl_pack(v0, v1);
+}
+__device__ __forceinline__ u64 gl_reduce5(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3,
+                                          uint32_t r4) {
+  const u64 v = gl_reduce_lazy(r0, r1, r2, r3, r4);
+  return gl_canon_words((uint32_t)v, (uint32_t)(v >> 32));
 }
 __device__ __forceinline__ u64 gl_reduce4(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
   return gl_reduce5(r0, r1, r2, r3, 0);
@@ -176,7 +181,13 @@ __device__ __forceinline__ u64 gl_acc_reduce(const Acc160& a) {
 #endif
 }
 #endif
-GL_HD u64 gl_canon(u64 a) { return a >= GL_P ? a - GL_P : a; }
+GL_HD u64 gl_canon(u64 a) {
+#ifdef __CUDA_ARCH__
+  return gl_canon_words((uint32_t)a, (uint32_t)(a >> 32));
+#else
+  return a >= GL_P ? a - GL_P : a;
+#endif
+}
 GL_HD u64 gl_pow(u64 a, u64 e) {
   u64 r = 1;
   while (e) {

@@ -18,10 +18,11 @@ void ntt_batch(const u64* in, size_t in_stride, size_t n_in, u64* out, size_t ou
 void transpose_u64(const u64* in, u64* out, size_t rows, size_t cols, size_t batch,
                    cudaStream_t st);
 
-// rs_dft.cu: the commitment rows' RS encoding for 2^RS_LOGN_MIN <= N <= 2^RS_LOGN_MAX, from N/2
-// (zero-padded) or N input values per row.  z: rows x N scratch.  tables: the context's
+// rs_dft.cu: row transforms (the commitment's RS encoding, Basefold's codewords) for
+// 2^RS_LOGN_MIN <= N <= 2^RS_LOGN_MAX from N/8, N/4, N/2 (zero-padded) or N input values per row,
+// any 64-bit representatives.  z: rows x N scratch (not used up to 2^13).  tables: the context's
 // rs_tables_elems() twiddles built by build_rs_tables from the main table.
-constexpr unsigned RS_LOGN_MIN = 14, RS_LOGN_MAX = 18;
+constexpr unsigned RS_LOGN_MIN = 12, RS_LOGN_MAX = 20;
 size_t rs_tables_elems();
 size_t rs_table_offset(unsigned logN);
 void build_rs_tables(u64* tables, const u64* tw, cudaStream_t st);

@@ -37,9 +37,7 @@ void bf_commit(lgs_ctx* c, const u64* poly, int is_ef, size_t len, unsigned li,
   u64* cT = ar.get<u64>(cols * L);
   u64* scr = logL > 12 ? ar.get<u64>(cols * L) : nullptr;
   transpose_u64(poly, tT, rows, cols, 1, st);
-  // large transforms use the row kernels (one CTA per four columns of a row, which fills the
-  // GPU only with many rows); the prove's small Basefold commits keep the Stockham kernels
-  if (rs_dft_supported(logL, rows) && cols * L >= ((size_t)1 << 22) && cols <= 65535)
+  if (rs_dft_supported(logL, rows))  // cols <= 128
     rs_dft_rows(tT, rows, rows, cT, L, logL, cols, scr, c->rs_tw.as<u64>(), st);
   else
     ntt_batch(tT, rows, rows, cT, L, logL, cols, scr, c->tw.as<u64>(), st);
@@ -1018,7 +1016,10 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
     u64* t2 = ar.get<u64>(2 * two_n);
     u64* scr = ilog2(two_n) > 12 ? ar.get<u64>(2 * two_n) : nullptr;
     transpose_u64((const u64*)a_vec, t1, n, 2, 1, b);
-    ntt_batch(t1, n, n, t2, two_n, ilog2(two_n), 2, scr, c->tw.as<u64>(), b);
+    if (rs_dft_supported(ilog2(two_n), n))
+      rs_dft_rows(t1, n, n, t2, two_n, ilog2(two_n), 2, scr, c->rs_tw.as<u64>(), b);
+    else
+      ntt_batch(t1, n, n, t2, two_n, ilog2(two_n), 2, scr, c->tw.as<u64>(), b);
     transpose_u64(t2, (u64*)ra, 2, two_n, 1, b);
     tl_mark("rs_end", b);
     y4_dev(eq_r2, ra, d_idx, S, (ef2*)(stage + S_y4), b);
