@@ -417,16 +417,6 @@ void eq_dot_multi_dev(const EqDotTask* tasks_dev, unsigned ntasks, unsigned k, e
   LGS_LAUNCH_CHECK();
 }
 
-__global__ void lift_bf_kernel(const u64* __restrict__ in, ef2* __restrict__ out, size_t n,
-                               u64 minus) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = ef_make(gl_sub(in[i], minus), 0);
-}
-void lift_bf(const u64* in, ef2* out, size_t n, u64 minus, cudaStream_t st) {
-  lift_bf_kernel<<<cdiv(n, 256), 256, 0, st>>>(in, out, n, minus);
-  LGS_LAUNCH_CHECK();
-}
-
 // ---- B_I: bi[i*s + k] = bit (i % 64) of F'[i / 64][idx[k]] (pcs/src/ligesis.rs:403-410) -----
 __global__ void bits_gather_kernel(const u64* const* __restrict__ cwref, size_t two_n,
                                    const uint64_t* __restrict__ idx, unsigned s, size_t rows,

@@ -81,9 +81,19 @@ size_t sumcheck_partials_elems(unsigned k, unsigned d);
 // max_blocks: grid cap of the multi-CTA passes (0 or above SC_MAX_BLOCKS: SC_MAX_BLOCKS).
 void sumcheck_prove_dev(ef2* const* polys, unsigned d, unsigned k, const ef2* ch, ef2* rounds_out,
                         ef2* final_out, ef2* partials, cudaStream_t st, unsigned max_blocks = 0);
-// The 3-factor sumcheck of [b, b - 1, eq] storing only b and eq (both folded in place).
-void sumcheck_binary_dev(ef2* b, ef2* eq, unsigned k, const ef2* ch, ef2* rounds_out,
-                         ef2* final_out, ef2* partials, cudaStream_t st, unsigned max_blocks = 0);
+// Up to SC_MAX_JOBS sumchecks of the same kind and size, launched together.  src is only read
+// (unless dst is src); dst[i] holds 2^(k-1) values of work space at most (k > 10; else unused).
+constexpr unsigned SC_MAX_JOBS = 2;
+struct ScJob {
+  const void* src[3];  // 2^k EF each; src[0] base-field words if bf0
+  ef2* dst[3];
+  const ef2* ch;
+  ef2 *rounds, *fin, *partials;
+  int bf0;
+  int binary;  // factors [b, b - 1, eq]: src[0] = b (0 or 1), src[1] = eq, d = 3
+};
+void sumcheck_jobs_dev(const ScJob* jobs, unsigned njobs, unsigned d, unsigned k, cudaStream_t st,
+                       unsigned max_blocks = 0);
 
 // eval.cu
 void canon_u64(u64* p, size_t n, cudaStream_t st);  // p[i] = p[i] mod p, in place
@@ -109,7 +119,6 @@ void eq_dot_dev(const void* vec, int is_bf, const ef2* point, unsigned k, ef2* o
 // a graph reads whichever buffer the slot names when it runs.
 void gemv_eq_rows(const u64* const* fref, const ef2* eq, size_t m, size_t n, ef2* out,
                   cudaStream_t st);
-void lift_bf(const u64* in, ef2* out, size_t n, u64 minus, cudaStream_t st);
 void bits_gather(const u64* const* cwref, size_t two_n, const uint64_t* idx, unsigned s,
                  size_t W, u64* bi, cudaStream_t st);
 void g1_build(const u64* const* aref, size_t W, const ef2* eq_a2, unsigned C, ef2* g1,

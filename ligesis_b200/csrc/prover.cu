@@ -910,7 +910,10 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
   // -- the transcript is a DAG of independent branches (every challenge is pre-drawn): fork them
   // onto side streams as soon as their inputs exist, join before the gather.  The branches that
   // need only B_I fork before the a-bar GEMV; the two Basefold commitments (A1, B) gate the
-  // Stage B codeword chain on the main stream and run on high-priority streams.
+  // Stage B codeword chain: A1 runs on the main stream, B on a high-priority one.  Short branches
+  // share a stream, so six chains run side by side: with ten, chains shared the hardware's work
+  // queues and waited for one another by chance (prove alone, six against ten: 2^3 x 2^11 145 us
+  // against 171, 2^6 x 2^14 240 against 276, 2^7 x 2^17 463 against 500, with the tiled sumchecks).
   new_eq_dev(d_prm + P_z1, s.log_m, eqz1, st);
   bits_gather(d_ptrs + PT_CW, two_n, d_idx, S, W, bi, st);
   new_eq_dev(d_fields + fp.alpha2, 5, eq_a2, st);
@@ -936,6 +939,13 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
   auto partials_for = [&](unsigned k, unsigned d) {
     return ar.get<ef2>(std::max(sumcheck_partials_elems(k, d), eqdot_partials_elems(k) + 1024));
   };
+  // challenges and results of sumcheck i of the proof
+  auto sc_job = [&](ScJob* j, unsigned ch, int i, ef2* partials) {
+    j->ch = d_fields + ch;
+    j->rounds = (ef2*)(stage + S_sc_r[i]);
+    j->fin = (ef2*)(stage + S_sc_f[i]);
+    j->partials = partials;
+  };
   const unsigned br_b = (unsigned)brs.size();
   // B: the Basefold commitment to B_I (pcs/src/ligesis.rs:411-416)
   {
@@ -944,18 +954,20 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
     bf_commit(c, bi, 0, WS, li_bi, CODE_RATE, &bi_st, b);
     mark("B_bi_commit_end", b);
   }
-  // C: binary check, factors [B_I, B_I - 1, eq_alpha1] (pcs/src/ligesis.rs:419-429); the
-  // longest branch, so it is the third high-priority one
+  // C: binary check, factors [B_I, B_I - 1, eq_alpha1] (pcs/src/ligesis.rs:419-429); the longest
+  // of the branches on B_I, so it is the other high-priority one
   {
     t_tl_branch = "C";
     cudaStream_t b = branch(true);
-    ef2* p0 = ar.get<ef2>(WS);
     ef2* p2 = ar.get<ef2>(WS);
-    lift_bf(bi, p0, WS, 0, b);
     new_eq_dev(d_fields + fp.alpha1, nb, p2, b);
     tl_mark("inputs_end", b);
-    sumcheck_binary_dev(p0, p2, nb, d_fields + fp.ch_bin, (ef2*)(stage + S_sc_r[0]),
-                        (ef2*)(stage + S_sc_f[0]), partials_for(nb, 3), b, c->sumcheck_blocks);
+    ScJob j{};
+    j.binary = j.bf0 = 1;
+    j.src[0] = bi, j.dst[0] = ar.get<ef2>(WS / 2);
+    j.src[1] = j.dst[1] = p2;
+    sc_job(&j, fp.ch_bin, 0, partials_for(nb, 3));
+    sumcheck_jobs_dev(&j, 1, 3, nb, b, c->sumcheck_blocks);
     mark("C_binary_sc_end", b);
   }
   // D: hash and recon bilinear sumchecks (pcs/src/ligesis.rs:435-485)
@@ -964,34 +976,34 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
     cudaStream_t b = branch();
     ef2* g1 = ar.get<ef2>(W);
     ef2* g2 = ar.get<ef2>(W);
-    ef2* g2b = ar.get<ef2>(W);
     ef2* v = ar.get<ef2>(W);
     g1_build(d_ptrs + PT_A, W, eq_a2, DIGEST_ROWS, g1, b);
     g2_build(bi, W, S, eq_r2, g2, b);
-    d2d(g2b, g2, W * sizeof(ef2), b);
     v_build(eqz1, W, v, b);
     tl_mark("inputs_end", b);
-    ef2* ph[2] = {g1, g2};
-    ef2* part = partials_for(log_w, 2);
-    sumcheck_prove_dev(ph, 2, log_w, d_fields + fp.ch_hash, (ef2*)(stage + S_sc_r[1]),
-                       (ef2*)(stage + S_sc_f[1]), part, b, c->sumcheck_blocks);
-    ef2* pr[2] = {v, g2b};
-    sumcheck_prove_dev(pr, 2, log_w, d_fields + fp.ch_recon, (ef2*)(stage + S_sc_r[2]),
-                       (ef2*)(stage + S_sc_f[2]), part, b, c->sumcheck_blocks);
+    ScJob j[2] = {};  // [g1, g2] and [v, g2], side by side
+    j[0].src[0] = j[0].dst[0] = g1;
+    j[1].src[0] = j[1].dst[0] = v;
+    for (int y = 0; y < 2; ++y) {
+      j[y].src[1] = g2, j[y].dst[1] = ar.get<ef2>(W / 2);
+      sc_job(&j[y], y ? fp.ch_recon : fp.ch_hash, 1 + y, partials_for(log_w, 2));
+    }
+    sumcheck_jobs_dev(j, 2, 2, log_w, b, c->sumcheck_blocks);
     mark("D_hash_recon_sc_end", b);
   }
   // F: Stage A point reduction of B_I (pcs/src/ligesis.rs:510-516)
   {
     t_tl_branch = "F";
-    cudaStream_t b = branch();
+    cudaStream_t b = brs.back();
     ef2* gbi = ar.get<ef2>(WS);
-    ef2* bie = ar.get<ef2>(WS);
     combine_eq_dev(d_prm + P_bipts, 3, nb, d_fields + fp.gamma_bi, gbi, b);
-    lift_bf(bi, bie, WS, 0, b);
     tl_mark("inputs_end", b);
-    ef2* pb[2] = {bie, gbi};
-    sumcheck_prove_dev(pb, 2, nb, d_fields + fp.ch_bi, (ef2*)(stage + S_sc_r[5]),
-                       (ef2*)(stage + S_sc_f[5]), partials_for(nb, 2), b, c->sumcheck_blocks);
+    ScJob j{};
+    j.bf0 = 1;
+    j.src[0] = bi, j.dst[0] = ar.get<ef2>(WS / 2);
+    j.src[1] = j.dst[1] = gbi;
+    sc_job(&j, fp.ch_bi, 5, partials_for(nb, 2));
+    sumcheck_jobs_dev(&j, 1, 2, nb, b, c->sumcheck_blocks);
     mark("F_bi_batch_sc_end", b);
   }
   // -- a-bar = eq_{z1}^T F and everything that needs it (pcs/src/ligesis.rs:365-387)
@@ -999,15 +1011,6 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
   mark("abar_end", st);
   LGS_CUDA(cudaEventRecord(c->ev_fork2, st));
   fork_ev = c->ev_fork2;
-  const unsigned br_a1 = (unsigned)brs.size();
-  // A1: y = a(z2) and the Basefold commitment to a-bar (pcs/src/ligesis.rs:379-384)
-  {
-    t_tl_branch = "A1";
-    cudaStream_t b = branch(true);
-    eq_dot_dev(a_vec, 0, d_prm + P_z2, log_n, (ef2*)(stage + S_y), partials_for(log_n, 1), b);
-    bf_commit(c, (const u64*)a_vec, 1, n, li_a, CODE_RATE, &a_st, b);
-    mark("A1_abar_commit_end", b);
-  }
   // A2: RS(a-bar), y4, the recon table sumcheck and y5 (pcs/src/ligesis.rs:387, 458, 487-497)
   {
     t_tl_branch = "A2";
@@ -1024,47 +1027,41 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
     tl_mark("rs_end", b);
     y4_dev(eq_r2, ra, d_idx, S, (ef2*)(stage + S_y4), b);
     ef2* sel = ar.get<ef2>(two_n);
-    ef2* rac = ar.get<ef2>(two_n);
     sel_build(d_idx, eq_r2, S, two_n, sel, b);
-    d2d(rac, ra, two_n * sizeof(ef2), b);
-    ef2* pt[2] = {sel, rac};
-    sumcheck_prove_dev(pt, 2, log_n + 1, d_fields + fp.ch_table, (ef2*)(stage + S_sc_r[3]),
-                       (ef2*)(stage + S_sc_f[3]), partials_for(log_n + 1, 2), b, c->sumcheck_blocks);
+    ScJob j{};
+    j.src[0] = j.dst[0] = sel;
+    j.src[1] = ra, j.dst[1] = ar.get<ef2>(n);
+    sc_job(&j, fp.ch_table, 3, partials_for(log_n + 1, 2));
+    sumcheck_jobs_dev(&j, 1, 2, log_n + 1, b, c->sumcheck_blocks);
     eq_dot_dev(ra, 0, d_prm + P_r3, log_n + 1, (ef2*)(stage + S_y5), partials_for(log_n + 1, 1), b);
     mark("A2_rs_abar_table_sc_end", b);
   }
-  // E: RS-link sumcheck (pcs/src/ligesis.rs:499-502); r3 is pre-drawn, so w needs no wait
+  // EG: the RS-link sumcheck (pcs/src/ligesis.rs:499-502; r3 is pre-drawn, so w needs no wait) and
+  // the Stage A point reduction of a-bar (:518-522), both on a-bar, side by side
   {
-    t_tl_branch = "E";
+    t_tl_branch = "EG";
     cudaStream_t b = branch();
     ef2* w = ar.get<ef2>(n);
-    ef2* ac = ar.get<ef2>(n);
-    rs_weights_dev(d_prm + P_r3, log_n + 1, n, c->tw.as<u64>(), w, b);
-    d2d(ac, a_vec, n * sizeof(ef2), b);
-    ef2* pw[2] = {ac, w};
-    sumcheck_prove_dev(pw, 2, log_n, d_fields + fp.ch_rs, (ef2*)(stage + S_sc_r[4]),
-                       (ef2*)(stage + S_sc_f[4]), partials_for(log_n, 2), b, c->sumcheck_blocks);
-    mark("E_rslink_sc_end", b);
-  }
-  // G: Stage A point reduction of a-bar (pcs/src/ligesis.rs:518-522)
-  {
-    t_tl_branch = "G";
-    cudaStream_t b = branch();
     ef2* ga = ar.get<ef2>(n);
-    ef2* ac = ar.get<ef2>(n);
+    rs_weights_dev(d_prm + P_r3, log_n + 1, n, c->tw.as<u64>(), w, b);
     combine_eq_dev(d_prm + P_apts, 2, log_n, d_fields + fp.gamma_a, ga, b);
-    d2d(ac, a_vec, n * sizeof(ef2), b);
-    ef2* pa[2] = {ac, ga};
-    sumcheck_prove_dev(pa, 2, log_n, d_fields + fp.ch_a, (ef2*)(stage + S_sc_r[6]),
-                       (ef2*)(stage + S_sc_f[6]), partials_for(log_n, 2), b, c->sumcheck_blocks);
-    mark("G_a_batch_sc_end", b);
+    ScJob j[2] = {};
+    j[0].src[1] = j[0].dst[1] = w;
+    j[1].src[1] = j[1].dst[1] = ga;
+    for (int y = 0; y < 2; ++y) {
+      j[y].src[0] = a_vec, j[y].dst[0] = ar.get<ef2>(n / 2);
+      sc_job(&j[y], y ? fp.ch_a : fp.ch_rs, y ? 6 : 4, partials_for(log_n, 2));
+    }
+    sumcheck_jobs_dev(j, 2, 2, log_n, b, c->sumcheck_blocks);
+    mark("EG_rslink_a_batch_sc_end", b);
   }
   // H: Stage B reduction messages (pcs/src/basefold.rs:746-769).  With m = poly.fold(point[0..li])
   // (2^R values) and the batch challenges r_0.., round t's l0 = MLE(m)(r_0, .., r_{t-1}, 0,
   // zp[t+1], .., zp[R-1]): the sequential rounds collapse to R independent evaluations.
   {
     t_tl_branch = "H";
-    cudaStream_t b = branch();
+    cudaStream_t b = brs.back();
+    eq_dot_dev(a_vec, 0, d_prm + P_z2, log_n, (ef2*)(stage + S_y), partials_for(log_n, 1), b);  // y
     const int poly_slot[3] = {PT_A, PT_BI, PT_AVEC};
     for (int ch = 0; ch < 3; ++ch)
       bf_fold_poly_dev(d_ptrs + poly_slot[ch], chan_ef[ch], chan_li[ch], pts[ch], mlen, mch[ch], b);
@@ -1072,10 +1069,13 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
     eq_dot_multi_dev((const EqDotTask*)(d_up + U_tasks), 3 * R, R, part, b);
     mark("H_basefold_msgs_end", b);
   }
+  // A1: the Basefold commitment to a-bar (pcs/src/ligesis.rs:379-384), on the main stream
+  t_tl_branch = "A1";
+  bf_commit(c, (const u64*)a_vec, 1, n, li_a, CODE_RATE, &a_st, st);
+  mark("A1_abar_commit_end", st);
   t_tl_branch = "main";
   // join: main waits for every branch
   for (size_t i = 0; i < brs.size(); ++i) LGS_CUDA(cudaEventRecord(c->ev_done[i], brs[i]));
-  LGS_CUDA(cudaStreamWaitEvent(st, c->ev_done[br_a1], 0));
   LGS_CUDA(cudaStreamWaitEvent(st, c->ev_done[br_b], 0));
   mark("main_suffix_start", st);
   // Stage B codeword chain on main (needs both prove-time commitments): combined level 0,
