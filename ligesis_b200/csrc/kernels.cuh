@@ -40,7 +40,7 @@ size_t tensor_map_bytes();
 void make_i64_tmap(const int64_t* base, size_t rows, size_t inner, unsigned box_rows,
                    void* tmap_out);
 // wait_cycles: clock budget of the kernel's bounded waits (0 = the default, about 2 s).
-// max_ctas: persistent CTAs (0 = one per SM); fewer leave SMs to concurrent work.
+// max_ctas: persistent CTAs, in pairs (0 = one per SM); fewer leave SMs to concurrent work.
 // Rows [row0, row0 + rows) of the codeword only (rows = 0: to the end; both even except at the
 // end): H is linear in the rows, so mode 0 writes the rows' partial digest, mode 1 adds it to H,
 // and modes 2 and 3 (write, add) also hash the finished H's leaves.
@@ -48,8 +48,8 @@ void subset_sum_hash_tc(const void* tmap, const u64* cw, u64* H, u32* leaves, un
                         size_t two_n, int* err, cudaStream_t st, uint64_t wait_cycles = 0,
                         unsigned max_ctas = 0, unsigned row0 = 0, unsigned rows = 0,
                         int mode = 2, u64* split_scratch = nullptr);
-// When the codeword has fewer 256-column tiles than CTAs, the hash splits its K rows over CTAs
-// into this many digest slices (a power of two); split_scratch must then hold splits x 32 x two_n
+// When the codeword's 256-column tiles do not fill the CTA pairs, the hash splits its K rows over
+// them into this many digest slices; split_scratch must then hold splits x 32 x two_n
 // values (splits == 1: none needed).
 unsigned subset_sum_hash_splits(size_t two_n, unsigned rows, unsigned max_ctas = 0);
 // Dense tcgen05 kind::i8 throughput (TOP/s) of back-to-back M128 N256 K32 MMAs on every SM.
