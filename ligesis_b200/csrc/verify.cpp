@@ -2,7 +2,6 @@
 // sumcheck::verify (utils/src/sumcheck.rs:88-130), Basefold::batch_verify
 // (pcs/src/basefold.rs:860-1035) and Merkle multiproof checks (utils/src/merkle.rs:89-103).
 // The verifier is cheap CPU work in the reference as well; it runs on the caller's thread.
-#include <map>
 #include <stdexcept>
 
 #include "blake3.cuh"
@@ -106,14 +105,19 @@ bool sc_verify(ef2 claim, const ScProof& p, Oracle& o, EFv* ch) {
   return ef_eq(prod, cur);
 }
 
-Hash32 hash_bytes(const std::vector<uint8_t>& b) {
-  u32 out[8];
+// Hash of a Merkle leaf: its words little-endian, which is how u64 and ef2 values lie in memory
+// on the hosts this library is built for.
+template <class F>
+Hash32 hash_leaf(const std::vector<F>& v) {
+  const uint8_t* b = (const uint8_t*)v.data();
   auto word = [&](u32 i) {
-    return (u32)b[4 * i] | ((u32)b[4 * i + 1] << 8) | ((u32)b[4 * i + 2] << 16) |
-           ((u32)b[4 * i + 3] << 24);
+    u32 w;
+    std::memcpy(&w, b + 4 * (size_t)i, 4);
+    return w;
   };
-  b3_hash_words(word, (u32)b.size(), out);
   Hash32 h;
+  u32 out[8];
+  b3_hash_words(word, (u32)(v.size() * sizeof(F)), out);
   std::memcpy(h.b, out, 32);
   return h;
 }
@@ -126,20 +130,6 @@ Hash32 hash_pair(const Hash32& l, const Hash32& r) {
   std::memcpy(h.b, o, 32);
   return h;
 }
-void ser(std::vector<uint8_t>& b, u64 v) {
-  for (int i = 0; i < 8; ++i) b.push_back((uint8_t)(v >> (8 * i)));
-}
-std::vector<uint8_t> leaf_bytes(const std::vector<u64>& v) {
-  std::vector<uint8_t> b;
-  for (u64 x : v) ser(b, x);
-  return b;
-}
-std::vector<uint8_t> leaf_bytes(const std::vector<ef2>& v) {
-  std::vector<uint8_t> b;
-  for (auto& x : v) ser(b, x.c0), ser(b, x.c1);
-  return b;
-}
-
 // rs_merkle root reconstruction from sorted distinct indices (power-of-two trees).
 bool merkle_check(const Hash32& root, const std::vector<uint8_t>& proof,
                   const std::vector<uint64_t>& idx, const std::vector<Hash32>& leaves,
@@ -148,28 +138,32 @@ bool merkle_check(const Hash32& root, const std::vector<uint8_t>& proof,
   if (nleaves == 0 || (nleaves & (nleaves - 1))) return false;
   for (size_t i = 0; i < idx.size(); ++i)
     if (idx[i] >= nleaves || (i && idx[i] <= idx[i - 1])) return false;
-  std::map<uint64_t, Hash32> known;
-  for (size_t i = 0; i < idx.size(); ++i) known[idx[i]] = leaves[i];
+  // the known nodes of a level in index order, replaced in place by their parents: the sibling that
+  // is missing comes from the proof, in the same order
+  std::vector<uint64_t> at(idx);
+  std::vector<Hash32> node(leaves);
   size_t pos = 0;
   for (uint64_t len = nleaves; len > 1; len >>= 1) {
-    std::vector<uint64_t> cur;
-    for (auto& kv : known) cur.push_back(kv.first);
-    for (uint64_t i : cur) {
-      uint64_t s = i ^ 1;
-      if (!known.count(s)) {
-        if (pos + 32 > proof.size()) return false;
-        Hash32 h;
-        std::memcpy(h.b, proof.data() + pos, 32);
+    size_t up = 0;
+    for (size_t i = 0; i < at.size(); ++up) {
+      const uint64_t p = at[i];
+      if (!(p & 1) && i + 1 < at.size() && at[i + 1] == p + 1) {
+        node[up] = hash_pair(node[i], node[i + 1]);
+        i += 2;
+      } else {
+        if (proof.size() - pos < 32) return false;
+        Hash32 s;
+        std::memcpy(s.b, proof.data() + pos, 32);
         pos += 32;
-        known[s] = h;
+        node[up] = p & 1 ? hash_pair(s, node[i]) : hash_pair(node[i], s);
+        i += 1;
       }
+      at[up] = p >> 1;
     }
-    std::map<uint64_t, Hash32> next;
-    for (auto& kv : known)
-      if (!(kv.first & 1)) next[kv.first / 2] = hash_pair(kv.second, known[kv.first + 1]);
-    known.swap(next);
+    at.resize(up);
+    node.resize(up);
   }
-  return pos == proof.size() && known.size() == 1 && known.begin()->second == root;
+  return pos == proof.size() && node[0] == root;
 }
 template <class F>
 bool opening_check(const OpeningH<F>& op, const Hash32& root, uint64_t nleaves) {
@@ -177,15 +171,21 @@ bool opening_check(const OpeningH<F>& op, const Hash32& root, uint64_t nleaves) 
   std::vector<Hash32> lh;
   for (auto& kv : op.values) {
     idx.push_back(kv.first);
-    lh.push_back(hash_bytes(leaf_bytes(kv.second)));
+    lh.push_back(hash_leaf(kv.second));
   }
   return merkle_check(root, op.proof, idx, lh, nleaves);
 }
 
-ef2 eq_fold_at(ef2 a, ef2 b, ef2 r, uint64_t len, uint64_t pos) {
-  u64 g = gl_two_adic_generator(ilog2_u64(len));
-  u64 tw = gl_pow(gl_inv(g), pos);
-  u64 inv2 = gl_inv(2);
+// The inverse of the generator of the order-len subgroup, len = d >> k, of every fold level k.
+std::vector<u64> level_inverses(uint64_t d, size_t rounds) {
+  std::vector<u64> v;
+  for (size_t k = 0; k < rounds; ++k)
+    v.push_back(gl_inv(gl_two_adic_generator(ilog2_u64(d >> k))));
+  return v;
+}
+ef2 eq_fold_at(ef2 a, ef2 b, ef2 r, u64 ginv, uint64_t pos) {
+  constexpr u64 inv2 = (GL_P + 1) / 2;
+  u64 tw = gl_pow(ginv, pos);
   ef2 pe = ef_scale(ef_add(a, b), inv2);
   ef2 po = ef_scale(ef_scale(ef_sub(a, b), tw), inv2);
   return ef_add(ef_mul(ef_sub(ef_one(), r), pe), ef_mul(r, po));
@@ -275,6 +275,7 @@ bool batch_verify(const std::vector<Claim>& bfc, const std::vector<Claim>& efc,
   };
   const uint64_t final_len = d >> rounds;
   if (pf.final_codeword.size() != final_len) return false;
+  const std::vector<u64> ginv = level_inverses(d, rounds);
   for (uint64_t idx : base) {
     bool have = false;
     ef2 der = ef_zero();
@@ -283,7 +284,7 @@ bool batch_verify(const std::vector<Claim>& bfc, const std::vector<Claim>& efc,
       ef2 a = val_at(k, pos), b = val_at(k, pos + half);
       if (!ok) return false;
       if (have && !ef_eq(der, (idx % cur) == pos ? a : b)) return false;
-      der = eq_fold_at(a, b, ch[k], cur, pos);
+      der = eq_fold_at(a, b, ch[k], ginv[k], pos);
       have = true;
     }
     if (have && !ef_eq(der, pf.final_codeword[idx % final_len])) return false;
@@ -363,6 +364,7 @@ int basefold_verify_host(const Hash32& root, const u64* point, size_t plen, cons
     };
     // fold consistency of every query down to the final codeword
     const uint64_t final_len = l >> rounds;
+    const std::vector<u64> ginv = level_inverses(l, rounds);
     for (uint64_t idx : base) {
       ef2 derived{};
       for (unsigned k = 0; k < rounds; ++k) {
@@ -370,7 +372,7 @@ int basefold_verify_host(const Hash32& root, const u64* point, size_t plen, cons
         ef2 a, b;
         if (!val_at(k, pos, &a) || !val_at(k, sib, &b)) return false;
         if (k > 0 && !ef_eq(derived, (idx % cur == pos) ? a : b)) return false;
-        derived = eq_fold_at(a, b, ch[k], cur, pos);
+        derived = eq_fold_at(a, b, ch[k], ginv[k], pos);
       }
       if (!ef_eq(derived, pf.final_codeword[idx % final_len])) return false;
     }
@@ -416,7 +418,7 @@ int verify_host(unsigned log_m, unsigned log_n, const Hash32& com_a, const Hash3
       if (col.size() != DIGEST_ROWS) return false;
     {
       std::vector<Hash32> lh;
-      for (auto& col : pf.h_cols) lh.push_back(hash_bytes(leaf_bytes(col)));
+      for (auto& col : pf.h_cols) lh.push_back(hash_leaf(col));
       if (!merkle_check(root, pf.h_open, sidx, lh, two_n)) return false;
     }
     {
@@ -463,20 +465,24 @@ int verify_host(unsigned log_m, unsigned log_n, const Hash32& com_a, const Hash3
       }
       if (!sc_verify(pf.y5, pf.sc[4], o, &ch)) return false;
       EFv r6 = rev(ch);
-      {  // w(r6), w[k] = prod_t (1 - r3[t] + r3[t] g^((2^t k) mod 2n))
+      {  // w(r6), w[k] = prod_t (1 - r3[t] + r3[t] g^((2^t k) mod 2n)): factor t depends on the
+         // low lg - t bits of k, and its sign alone on the highest of them, so the products over
+         // t >= T double in length as T falls: 2n products in F_p2 instead of n lg
         const unsigned lg = ilog2_u64(two_n);
         const u64 g = gl_two_adic_generator(lg);
-        std::vector<u64> gt(two_n);  // g^e for e < 2n
+        std::vector<u64> gt(n);  // g^e for e < n
         gt[0] = 1;
-        for (uint64_t e = 1; e < two_n; ++e) gt[e] = gl_mul(gt[e - 1], g);
+        for (uint64_t e = 1; e < n; ++e) gt[e] = gl_mul(gt[e - 1], g);
         EFv w(n);
-        for (uint64_t k = 0; k < n; ++k) {
-          ef2 prod = ef_one();
-          for (unsigned t = 0; t < lg; ++t) {
-            u64 gv = gt[(k << t) & (two_n - 1)];
-            prod = ef_mul(prod, ef_add(ef_sub(ef_one(), r3[t]), ef_scale(r3[t], gv)));
+        w[0] = ef_one();
+        for (unsigned t = lg; t-- > 0;) {
+          const uint64_t half = two_n >> (t + 1);
+          for (uint64_t k = 0; k < half; ++k) {
+            const ef2 ar = ef_mul(w[k], r3[t]), u = ef_sub(w[k], ar);
+            const ef2 v = ef_scale(ar, gt[k << t]);
+            if (half < n) w[k + half] = ef_sub(u, v);
+            w[k] = ef_add(u, v);
           }
-          w[k] = prod;
         }
         if (pf.sc[4].finals.size() != 2 || !ef_eq(pf.sc[4].finals[1], mle_eval(w, r6))) return false;
       }
