@@ -196,6 +196,22 @@ lgs_status lgs_softmax_witness(lgs_ctx* ctx, const int64_t* scores, unsigned hea
  * outside the table gives LGS_ERR_BAD_SHAPE. */
 lgs_status lgs_lut_gather(lgs_ctx* ctx, const int64_t* v, size_t count, const int64_t* lut,
                           size_t lut_len, int64_t offset, int on_device, int64_t* out);
+/* One block of the integer GPT-2 forward (model.rs:213-221): layer norm, attention, layer norm and
+ * MLP of the calls above, from host arrays, with nothing leaving the device in between.  X is n x
+ * d, n the sequence length (d = heads x the head size); weights: ln_1 gain and bias, attn_w (d x 3d)
+ * and bias, attn_proj_w (d x d) and bias, ln_2 gain and bias, fc_w (d x hidden) and bias, fproj_w
+ * (hidden x d) and bias.  score_scale divides the scores, scale everything else; offset moves
+ * both tables' indices.  out receives 36 arrays, each starting at a multiple of 32 values: ln1
+ * (sum_x, sum_x2, var_sum, std, dividend, quotient, output), attention (q_qkv, qkv, scores, x_max,
+ * exp, sum_exp, prob, heads' outputs, merged outputs, q_proj, X + proj, and the remainders of qkv,
+ * scores, heads' outputs, proj), ln2 (as ln1), MLP (q_fc, fc, act, q_fproj, X_out, and the
+ * remainders of fc, fproj).  *done = 0, with out not written, when a value needs the calls above
+ * one by one (operands outside the tensor-core encodings, or an error that they report). */
+lgs_status lgs_block_witness(lgs_ctx* ctx, const int64_t* x, unsigned n, unsigned d, unsigned heads,
+                             unsigned hidden, const int64_t* const weights[12],
+                             const int64_t* exp_lut, size_t exp_len, const int64_t* gelu_lut,
+                             size_t gelu_len, int64_t scale, int64_t score_scale, int64_t offset,
+                             int64_t* out, int* done);
 
 /* ---- batched and served proving (the reference proves one polynomial at a time on one
  * thread, pcs/benches/ligesis.rs:20-60) ----

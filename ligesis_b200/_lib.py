@@ -106,6 +106,9 @@ _SIGS = {
                                       C.c_int64, C.c_int, i64p, i64p, i64p, i64p]),
     "lgs_lut_gather": (C.c_int, [vp, i64p, C.c_size_t, i64p, C.c_size_t, C.c_int64, C.c_int,
                                  i64p]),
+    "lgs_block_witness": (C.c_int, [vp, i64p, C.c_uint, C.c_uint, C.c_uint, C.c_uint,
+                                    C.POINTER(i64p), i64p, C.c_size_t, i64p, C.c_size_t,
+                                    C.c_int64, C.c_int64, C.c_int64, i64p, C.POINTER(C.c_int)]),
     "lgs_tensor_peak_i8": (C.c_int, [vp, C.c_uint, C.POINTER(C.c_double)]),
     "lgs_rs_alu_rates": (C.c_int, [vp, C.c_uint, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "lgs_dft": (C.c_int, [vp, u64p, C.c_size_t, C.c_size_t, C.c_uint, u64p]),

@@ -502,6 +502,21 @@ lgs_status lgs_lut_gather(lgs_ctx* ctx, const int64_t* v, size_t count, const in
   });
 }
 
+lgs_status lgs_block_witness(lgs_ctx* ctx, const int64_t* x, unsigned n, unsigned d, unsigned heads,
+                             unsigned hidden, const int64_t* const weights[12],
+                             const int64_t* exp_lut, size_t exp_len, const int64_t* gelu_lut,
+                             size_t gelu_len, int64_t scale, int64_t score_scale, int64_t offset,
+                             int64_t* out, int* done) {
+  return guarded([&] {
+    need(ctx && x && weights && exp_lut && gelu_lut && out && done,
+         "lgs_block_witness: null argument");
+    for (int i = 0; i < 12; ++i) need(weights[i] != nullptr, "lgs_block_witness: null weights");
+    CtxDevice dg(ctx);
+    *done = block_witness_dev(ctx, x, n, d, heads, hidden, weights, exp_lut, exp_len, gelu_lut,
+                              gelu_len, scale, score_scale, offset, out);
+  });
+}
+
 lgs_status lgs_basefold_verify(const uint8_t root[32], const uint64_t* point, size_t plen,
                                const uint8_t* proof, size_t proof_len, const uint64_t* fields,
                                size_t nfields, const uint64_t* ints, size_t nints,

@@ -156,6 +156,33 @@ void h2d_staged(lgs_ctx* c, void* dst, const void* src, size_t bytes, cudaStream
   }
 }
 
+// Device-to-host copy of a large array into pageable memory through the same ring: the copy pool
+// empties chunk i - 1 while the DMA engine fills chunk i.  Returns once the array is complete.
+void d2h_staged(lgs_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  constexpr size_t CHUNK = lgs_ctx::RING_CHUNK / 2;
+  auto empty = [&](unsigned slot, size_t off) {
+    const size_t len = std::min(CHUNK, bytes - off);
+    LGS_CUDA(cudaEventSynchronize(c->ring_ev[slot]));
+    if (c->copy_pool)
+      CopyPool::get().copy((char*)dst + off, c->ring[slot].p, len);
+    else
+      std::memcpy((char*)dst + off, c->ring[slot].p, len);
+  };
+  unsigned prev = 0;
+  for (size_t off = 0; off < bytes; off += CHUNK) {
+    const unsigned slot = c->ring_next++ % lgs_ctx::RING;
+    const size_t len = std::min(CHUNK, bytes - off);
+    LGS_CUDA(cudaEventSynchronize(c->ring_ev[slot]));
+    c->ring[slot].reserve(lgs_ctx::RING_CHUNK);
+    LGS_CUDA(cudaMemcpyAsync(c->ring[slot].p, (const char*)src + off, len, cudaMemcpyDeviceToHost,
+                             st));
+    LGS_CUDA(cudaEventRecord(c->ring_ev[slot], st));
+    if (off) empty(prev, off - CHUNK);
+    prev = slot;
+  }
+  if (bytes) empty(prev, (bytes - 1) / CHUNK * CHUNK);
+}
+
 namespace {
 
 Hash32 read_root(const u32* nodes, size_t nleaves, cudaStream_t st) {

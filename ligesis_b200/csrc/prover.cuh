@@ -358,6 +358,7 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
                size_t nints, uint64_t cursors[2], std::vector<uint8_t>* proof_out);
 // Host-to-device copy of a (pageable) host buffer through the context's pinned ring.
 void h2d_staged(lgs_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t st);
+void d2h_staged(lgs_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t st);
 // GKR fraction sum (logup/src/frac_sum.rs:110-161) and GKR-LogUp lookup
 // (logup/src/lookup.rs:119-143) on the device (frac_sum.cu), proofs encoded "LGSF" / "LGSL"; and
 // their host verifiers (logup_verify.cpp).  Inputs are EF arrays (2 u64 per value) on the host,
@@ -396,6 +397,12 @@ void softmax_witness_dev(lgs_ctx* c, const int64_t* scores, unsigned heads, unsi
                          int64_t* prob);
 void lut_gather_dev(lgs_ctx* c, const int64_t* v, size_t count, const int64_t* lut,
                     size_t lut_len, int64_t offset, bool on_device, int64_t* out);
+// One whole transformer block of the witness from host arrays (witness.cu); false when the layers
+// have to be run one by one.
+bool block_witness_dev(lgs_ctx* c, const int64_t* x, unsigned n, unsigned d, unsigned heads,
+                       unsigned hidden, const int64_t* const w[12], const int64_t* exp_lut,
+                       size_t exp_len, const int64_t* gelu_lut, size_t gelu_len, int64_t scale,
+                       int64_t score_scale, int64_t offset, int64_t* out);
 lgs_status set_error(lgs_status s, const std::string& msg);
 lgs_status status_of_current_exception();
 }  // namespace lgs

@@ -610,4 +610,165 @@ void lut_gather_dev(lgs_ctx* c, const int64_t* v, size_t count, const int64_t* l
             });
 }
 
+// ---- one block of the integer GPT-2 (model.rs:213-221) without leaving the device ----
+namespace {
+
+// Per-head scores, floor_div(q_h k_h^T, divisor), of the rows x 3d output of the qkv layer (head h
+// in columns h dh .. of each third).  A thread per entry with an exact 128-bit sum: n^2 heads
+// products of dh terms are microseconds of work, and 12 separate linear layers of 31 x 64 x 31
+// were 12 times a call's launches, copies and waits.
+__global__ void head_scores_kernel(const int64_t* __restrict__ qkv, unsigned heads, unsigned n,
+                                   unsigned dh, int64_t divisor, int64_t* __restrict__ q,
+                                   int64_t* __restrict__ rem, int* __restrict__ err) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (size_t)heads * n * n) return;
+  const size_t j = t % n, i = t / n % n, h = t / ((size_t)n * n), d = (size_t)heads * dh;
+  const int64_t *a = qkv + i * 3 * d + h * dh, *b = qkv + j * 3 * d + d + h * dh;
+  Acc128 s{0, 0};
+  for (unsigned k = 0; k < dh; ++k) mac128(s, a[k], b[k]);
+  if (!lw_finish(s, nullptr, 0, divisor, t, q, rem, q, nullptr)) atomicOr(err, 1);
+}
+
+// Per-head weighted values, floor_div(prob_h v_h, divisor), in head order and merged to n x d rows.
+__global__ void head_values_kernel(const int64_t* __restrict__ prob,
+                                   const int64_t* __restrict__ qkv, unsigned heads, unsigned n,
+                                   unsigned dh, int64_t divisor, int64_t* __restrict__ q,
+                                   int64_t* __restrict__ rem, int64_t* __restrict__ merged,
+                                   int* __restrict__ err) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (size_t)heads * n * dh) return;
+  const size_t e = t % dh, i = t / dh % n, h = t / ((size_t)dh * n), d = (size_t)heads * dh;
+  const int64_t *a = prob + (h * n + i) * n, *b = qkv + 2 * d + h * dh + e;
+  Acc128 s{0, 0};
+  for (unsigned k = 0; k < n; ++k) mac128(s, a[k], b[(size_t)k * 3 * d]);
+  if (lw_finish(s, nullptr, 0, divisor, t, q, rem, q, nullptr))
+    merged[i * d + h * dh + e] = q[t];
+  else
+    atomicOr(err, 1);
+}
+
+__global__ void add_i64_kernel(const int64_t* __restrict__ a, const int64_t* __restrict__ b,
+                               int64_t* __restrict__ out, size_t count) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < count) out[i] = (int64_t)((uint64_t)a[i] + (uint64_t)b[i]);  // wraps
+}
+
+}  // namespace
+
+// The whole block from host arrays in one pass: every layer is enqueued as soon as its weights are
+// staged, so the uploads (77 MB at GPT-2's sizes, most of the time) run under the layers before
+// them; nothing waits in between, and the results leave in one copy.  Layer by layer it was 34
+// calls, each uploading its inputs, waiting, and reading pageable results back (31 x 768, 12 heads,
+// hidden 3072: 13.9 -> 4.8 ms; the bytes alone take 1.5 ms of PCIe).  False, with
+// nothing written, when a value needs the layer-by-layer path: operands outside the tensor-core
+// encodings, or a range error that path reports.
+bool block_witness_dev(lgs_ctx* c, const int64_t* x, unsigned n, unsigned d, unsigned heads,
+                       unsigned hidden, const int64_t* const w[12], const int64_t* exp_lut,
+                       size_t exp_len, const int64_t* gelu_lut, size_t gelu_len, int64_t scale,
+                       int64_t score_scale, int64_t offset, int64_t* out) {
+  if (c->witness_path != 0 || !n || !d || !heads || !hidden || d % heads || !exp_len ||
+      !gelu_len || scale <= 0 || score_scale <= 0 || n > 65536 || d > (1u << 22) ||
+      hidden > (1u << 24) || (size_t)heads * n > ((size_t)1 << 24))
+    return false;
+  cudaStream_t st = c->st;
+  Arena& ar = c->arena;
+  ar.begin();
+  const unsigned dh = d / heads;
+  const size_t nd = (size_t)n * d, nq = 3 * nd, nh = (size_t)n * hidden;
+  const size_t hn = (size_t)heads * n, hnn = hn * n;
+  // the fields in the order and at the offsets the caller reads them: each at a multiple of 32
+  const size_t size[36] = {
+      n,  n,  n,   n,  nd,  nd, nd,  // ln1: sum_x, sum_x2, var_sum, std, dividend, quotient, output
+      nq, nq, hnn, hn, hnn, hn, hnn, nd, nd, nd, nd, nq, hnn, nd, nd,  // attention
+      n,  n,  n,   n,  nd,  nd, nd,                                   // ln2
+      nh, nh, nh,  nd, nd,  nh, nd};                                  // mlp
+  size_t off[37] = {0};
+  for (int i = 0; i < 36; ++i) off[i + 1] = off[i] + (size[i] + 31) / 32 * 32;
+  int64_t* o = ar.get<int64_t>(off[36]);
+  auto fld = [&](int i) { return o + off[i]; };
+  constexpr int NERR = 16;  // two words per linear layer (8), then one per other step
+  int* derr = ar.get<int>(NERR);
+  LGS_CUDA(cudaMemsetAsync(derr, 0, NERR * sizeof(int), st));
+  // Uploads go on a stream of their own, so that a ring slot is free as soon as its copy is done
+  // and not behind the layers enqueued before it (8.3 -> 4.8 ms per block).
+  cudaStream_t cp = c->side[0];
+  LGS_CUDA(cudaEventRecord(c->ev_fork, st));  // the arena's earlier users are on the stream
+  LGS_CUDA(cudaStreamWaitEvent(cp, c->ev_fork, 0));
+  unsigned nup = 0;
+  auto in = [&](const int64_t* h, size_t count) {
+    int64_t* v = ar.get<int64_t>(count);
+    h2d_staged(c, v, h, count * 8, cp);
+    cudaEvent_t ev = c->ev_rows[nup++ % lgs_ctx::ROW_BLOCKS];
+    LGS_CUDA(cudaEventRecord(ev, cp));
+    LGS_CUDA(cudaStreamWaitEvent(st, ev, 0));
+    return v;
+  };
+  // the input and the vectors first, in one copy
+  const std::pair<const int64_t*, size_t> vecs[9] = {
+      {x, nd}, {w[0], d}, {w[1], d}, {w[3], 3 * (size_t)d}, {w[5], d}, {w[6], d}, {w[7], d},
+      {w[9], hidden}, {w[11], d}};
+  std::vector<int64_t> pack;
+  size_t at[9];
+  for (int i = 0; i < 9; ++i) {
+    at[i] = pack.size();
+    pack.insert(pack.end(), vecs[i].first, vecs[i].first + vecs[i].second);
+  }
+  const int64_t* dv = in(pack.data(), pack.size());
+  auto layer_norm = [&](const int64_t* xin, int g, int f, int* err) {
+    LnArgs a{xin, dv + at[g], dv + at[g + 1], n, d, fld(f), fld(f + 1), fld(f + 2), fld(f + 3),
+             fld(f + 4), fld(f + 5), fld(f + 6), err};
+    layer_norm_witness_kernel<<<n, 256, 0, st>>>(a);
+    LGS_LAUNCH_CHECK();
+  };
+  auto linear = [&](const int64_t* xin, size_t inner, const int64_t* wt, int b, size_t cols,
+                    int64_t* q, int64_t* rem, int64_t* y, int* err) {
+    const int64_t* dw = in(wt, inner * cols);
+    linear_witness_tc(c, xin, n, inner, dw, cols, false, dv + at[b], scale, q, rem, y, nullptr,
+                      err, err + 1);
+  };
+  auto add = [&](const int64_t* a, const int64_t* b, int64_t* r) {
+    add_i64_kernel<<<(unsigned)((nd + 255) / 256), 256, 0, st>>>(a, b, r, nd);
+    LGS_LAUNCH_CHECK();
+  };
+  int64_t* tmp = ar.get<int64_t>(nd);
+  // attention: fields 7 q_qkv, qkv, scores, x_max, exp, sum_exp, q_prob, q_ao_heads, q_ao, q_apr,
+  // x_out, rem_qkv, rem_sc, rem_ao_heads, rem_apr
+  const int64_t* dx = dv;
+  layer_norm(dx, 1, 0, derr + 8);
+  linear(fld(6), d, w[2], 3, 3 * (size_t)d, fld(7), fld(18), fld(8), derr);
+  head_scores_kernel<<<(unsigned)((hnn + 127) / 128), 128, 0, st>>>(
+      fld(8), heads, n, dh, score_scale, fld(9), fld(19), derr + 9);
+  LGS_LAUNCH_CHECK();
+  const int64_t* dexp = in(exp_lut, exp_len);
+  softmax_witness_kernel<<<(unsigned)((hn + 127) / 128), 128, 0, st>>>(
+      fld(9), heads, n, dexp, exp_len, offset, scale, fld(10), fld(11), fld(12), fld(13),
+      derr + 10);
+  LGS_LAUNCH_CHECK();
+  head_values_kernel<<<(unsigned)((nd + 127) / 128), 128, 0, st>>>(
+      fld(13), fld(8), heads, n, dh, scale, fld(14), fld(20), fld(15), derr + 11);
+  LGS_LAUNCH_CHECK();
+  linear(fld(15), d, w[4], 4, d, fld(16), fld(21), tmp, derr + 2);
+  add(dx, tmp, fld(17));
+  // mlp: fields 29 q_fc, fc, act, q_fpr, x_out, rem_fc, rem_fpr
+  layer_norm(fld(17), 5, 22, derr + 12);
+  linear(fld(28), d, w[8], 7, hidden, fld(29), fld(34), fld(30), derr + 4);
+  const int64_t* dgelu = in(gelu_lut, gelu_len);
+  lut_gather_kernel<<<(unsigned)std::min<size_t>((nh + 255) / 256, 148 * 8), 256, 0, st>>>(
+      fld(30), nh, dgelu, gelu_len, offset, fld(31), derr + 13);
+  LGS_LAUNCH_CHECK();
+  linear(fld(31), hidden, w[10], 8, d, fld(32), fld(35), tmp, derr + 6);
+  add(fld(17), tmp, fld(33));
+  int err[NERR];
+  LGS_CUDA(cudaMemcpyAsync(err, derr, sizeof(err), cudaMemcpyDeviceToHost, st));
+  LGS_CUDA(cudaStreamSynchronize(st));
+  for (int i = 0; i < 8; i += 2)
+    if (err[i] >= 16)
+      throw DeviceTimeout("linear witness: a bounded device wait gave up (code " +
+                          std::to_string(err[i]) + ")");
+  for (int e : err)
+    if (e) return false;
+  d2h_staged(c, out, o, off[36] * 8, st);
+  return true;
+}
+
 }  // namespace lgs

@@ -153,6 +153,44 @@ WEIGHT_NAMES = ("ln_1_g", "ln_1_b", "attn_w", "attn_b", "attn_proj_w", "attn_pro
                 "ln_2_b", "fc_w", "fc_b", "fproj_w", "fproj_b")
 
 
+def _block_on_device(x, w: dict, exp_lut, gelu_lut, cfg: dict, ctx: Context):
+    """`block_witness` as one native call (lgs_block_witness), or None where the layers are run one
+    by one: arrays that are not the block's plain shapes, or values that call leaves to them."""
+    n, d = cfg["n_seq"], cfg["d_model"]
+    H = cfg.get("n_head", 12)
+    host = lambda a: np.ascontiguousarray(a, dtype=np.int64)
+    ws = [host(w[k]) for k in WEIGHT_NAMES]
+    hid = ws[8].shape[-1]
+    shapes = [(d,), (d,), (d, 3 * d), (3 * d,), (d, d), (d,), (d,), (d,), (d, hid), (hid,),
+              (hid, d), (d,)]
+    luts = host(exp_lut), host(gelu_lut)
+    if (min(n, d, H, hid) < 1 or d % H or x.shape != (n, d) or any(t.ndim != 1 for t in luts)
+            or [a.shape for a in ws] != shapes):
+        return None
+    dh, sc = d // H, cfg["scale"]
+    ln = [(n,)] * 4 + [(n, d)] * 3
+    heads, merged = (H, n, n), (n, d)
+    attn = [(n, 3 * d)] * 2 + [heads, (H, n), heads, (H, n), heads, (H, n, dh), merged, merged,
+                               merged, (n, 3 * d), heads, (H, n, dh), merged]
+    mlp = [(n, hid)] * 3 + [merged] * 2 + [(n, hid), merged]
+    fields, off = [], 0
+    for shape in ln + attn + ln + mlp:
+        size = int(np.prod(shape))
+        fields.append((off, size, shape))
+        off += (size + 31) // 32 * 32
+    out = np.empty(off, np.int64)
+    p = lambda a: a.ctypes.data_as(i64p)
+    done = C.c_int(0)
+    check(load().lgs_block_witness(ctx.handle, p(x), n, d, H, hid, (i64p * 12)(*map(p, ws)),
+                                   p(luts[0]), luts[0].size, p(luts[1]), luts[1].size, sc,
+                                   sc * int(round(dh ** 0.5)), cfg["max_v"] * sc, p(out),
+                                   C.byref(done)))
+    if not done.value:
+        return None
+    return {f: out[o:o + size].reshape(shape)
+            for f, (o, size, shape) in zip(BLOCK_FIELDS, fields)}
+
+
 def block_witness(x, w: dict, exp_lut, gelu_lut, cfg: dict = GPT2_31,
                   ctx: Context | None = None) -> dict:
     """One block of the integer GPT-2 forward (model.rs:213-221): ln1, attention (qkv, per-head
@@ -167,6 +205,10 @@ def block_witness(x, w: dict, exp_lut, gelu_lut, cfg: dict = GPT2_31,
     sqrt_d_scale = sc * int(round(dh ** 0.5))  # Config::sqrt_d_scale (witness.rs:33-35)
     offset = cfg["max_v"] * sc
     x = np.ascontiguousarray(x, dtype=np.int64)
+    ctx = ctx or Context.default()
+    out = _block_on_device(x, w, exp_lut, gelu_lut, cfg, ctx)
+    if out is not None:
+        return out
     out = {}
     ln1 = layer_norm_witness(x, w["ln_1_g"], w["ln_1_b"], ctx)
     out.update({"ln1." + f: v for f, v in zip(LN_FIELDS, ln1)})
