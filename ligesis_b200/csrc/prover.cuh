@@ -274,6 +274,7 @@ struct lgs_ctx {
   unsigned hash_ctas = 0;        // persistent CTAs of the subset-sum hash (default: one per SM)
   unsigned sumcheck_blocks = 0;  // grid cap of the multi-CTA sumcheck passes (<= SC_MAX_BLOCKS)
   unsigned hash_groups = 0;      // host-rows commit: hash launches over row groups (0: default)
+  lgs::PinnedBuf wit_flags;  // the linear witness' error words, zero between calls
   unsigned witness_path = 0;     // linear witness: 0 tensor cores when the operands fit, 1 CUDA cores
   unsigned witness_ctas = 0;     // linear witness: resident CTAs its work plan assumes (0: the GPU's)
   size_t upload_block = 0;       // host-rows commit: least bytes per row block (0: 1 MB)

@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(256, 2) linear_witness_kernel(const LwArgs a) 
       else
         a.part[(size_t)blockIdx.z * a.rows * a.cols + o] = acc[i][j];
     }
-  if (bad) atomicOr(a.err, 1);
+  if (bad) set_err(a.err);
 }
 
 // Sums the K splits of every output (exactly) and finishes it.
@@ -255,7 +255,7 @@ __global__ void linear_witness_finish_kernel(const LwArgs a, unsigned nsplit) {
     for (unsigned z = 0; z < nsplit; ++z) add128(s, a.part[(size_t)z * n + o]);
     bad |= !lw_finish(s, a.bias, o % a.cols, a.d, o, a.q, a.rem, a.y, a.yf);
   }
-  if (bad) atomicOr(a.err, 1);
+  if (bad) set_err(a.err);
 }
 
 // layer_norm (proofsys/src/model.rs:241-279), one CTA per row: exact 128-bit sums of x and x^2,
@@ -368,23 +368,31 @@ void linear_witness_dev(lgs_ctx* c, const int64_t* x, size_t rows, size_t inner,
     dy = ar.get<int64_t>(no);
     df = y_field ? ar.get<uint64_t>(no) : nullptr;
   }
-  int* derr = ar.get<int>(2);  // error word, then the tensor path's operand-range flag
-  LGS_CUDA(cudaMemsetAsync(derr, 0, 2 * sizeof(int), st));
+  // Error word, then the tensor path's operand-range flag, in pinned memory that the kernels reach:
+  // they write it only when something is wrong, so a call needs no memset and no copy for it, and
+  // its one wait is the stream's (vocabulary head 119 -> 108 us a call, 1 x 32 x 32: 84 -> 67).
+  if (!c->wit_flags.p) {
+    c->wit_flags.reserve(2 * sizeof(int));
+    std::memset(c->wit_flags.p, 0, 2 * sizeof(int));
+  }
+  int* derr = c->wit_flags.as<int>();
+  int flags[2];
+  auto read_flags = [&] {
+    LGS_CUDA(cudaStreamSynchronize(st));
+    for (int i = 0; i < 2; ++i) flags[i] = ((volatile int*)derr)[i], derr[i] = 0;
+  };
   int herr = 0;
   bool done = false;
   if (c->witness_path == 0) {
     // operands within the limb encodings (every integer GPT-2 layer): the tensor cores
     linear_witness_tc(c, dx, rows, inner, dw, cols, w_transposed, db, divisor, dq, dr, dy, df,
                       derr, derr + 1);
-    int flags[2] = {0, 0};
-    LGS_CUDA(cudaMemcpyAsync(flags, derr, sizeof(flags), cudaMemcpyDeviceToHost, st));
-    LGS_CUDA(cudaStreamSynchronize(st));
+    read_flags();
     if (flags[0] >= 16)
       throw DeviceTimeout("linear witness: a bounded device wait gave up (code " +
                           std::to_string(flags[0]) + ")");
     done = flags[1] == 0;  // else an operand needs more than its limbs: the CUDA-core kernel
     if (done) herr = flags[0];
-    else LGS_CUDA(cudaMemsetAsync(derr, 0, 2 * sizeof(int), st));
   }
   if (!done) {
   // Few rows (GPT-2 runs 31 positions) leave most SMs idle: split K until there are about two
@@ -418,15 +426,16 @@ void linear_witness_dev(lgs_ctx* c, const int64_t* x, size_t rows, size_t inner,
     linear_witness_finish_kernel<<<blocks, 256, 0, st>>>(a, (unsigned)split);
     LGS_LAUNCH_CHECK();
   }
-  LGS_CUDA(cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  read_flags();
+  herr = flags[0];
   }
   if (!on_device) {
     LGS_CUDA(cudaMemcpyAsync(q, dq, no * 8, cudaMemcpyDeviceToHost, st));
     LGS_CUDA(cudaMemcpyAsync(rem, dr, no * 8, cudaMemcpyDeviceToHost, st));
     LGS_CUDA(cudaMemcpyAsync(y, dy, no * 8, cudaMemcpyDeviceToHost, st));
     if (y_field) LGS_CUDA(cudaMemcpyAsync(y_field, df, no * 8, cudaMemcpyDeviceToHost, st));
+    LGS_CUDA(cudaStreamSynchronize(st));
   }
-  LGS_CUDA(cudaStreamSynchronize(st));
   if (herr) throw ShapeError("linear witness: a product or Q + bias leaves the i64 range");
 }
 

@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(256) x_limbs_kernel(const WtArgs a, uint8_t* _
     if (lane == 0) xsum[(tile * chunks + chunk) * nr + r] = 0;
   }
   store_row<WT_LX>(tiles, r, e[0], e[1], e[2], e[3]);
-  if (bad) atomicExch(a.range, 1);
+  if (bad) set_flag(a.range);
 }
 
 // What the producer loop shares with the rest of its CTA.
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(WT_THREADS, 2) linear_witness_tc_kernel(const 
     const bool edge = c0 + WT_M > a.cols || (ke - kb) % WT_KC != 0;
     const uint64_t acc = edge ? wt_produce<WT, true>(a, cs) : wt_produce<WT, false>(a, cs);
     x_issued = cs.x_issued;
-    if (acc >> 16) atomicExch(a.range, 1);
+    if (acc >> 16) set_flag(a.range);
     // this CTA's sums of x' per row, from the per-chunk sums
     if (tid < nr) {
       unsigned long long sum = 0;
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(WT_THREADS, 2) linear_witness_tc_kernel(const 
         if (!s_fail) tc::flag_failure(&s_fail, a.err, 19);
       } else {
         if (!wt_epilogue(a, wu, tmem, sx, warp, 0, 1, lane, tid == 0, &s_last, 0))
-          atomicOr(a.err, 1);
+          set_err(a.err);
       }
     }
   }
@@ -798,7 +798,7 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
         if (lane == 0) tc::mbar_arrive(lim_full(s));
       }
     }
-    if (acc >> 16) atomicExch(a.range, 1);
+    if (acc >> 16) set_flag(a.range);
     if (tid == 0) {
       // the newest X copy of each stage may still be in flight: wait for it before exiting
       for (unsigned g = x_issued > WT_STAGES ? x_issued - WT_STAGES : 0; g < x_issued; ++g)
@@ -916,7 +916,7 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
       const int64_t wpad = (int64_t)((size_t)w.nch * WT_KC - (w.ke - w.kb)) << 15;
       if (!wt_epilogue(a, w, tmem + b * WT_NG * nr, sx, q, h, WP_EPI_HALVES, lane, et == 0, &s_last,
                        wpad))
-        atomicOr(a.err, 1);
+        set_err(a.err);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(acc_empty(b));
