@@ -13,6 +13,9 @@ constexpr unsigned SC_MAX_BLOCKS = 296;  // 2 CTAs per SM on a 148-SM B200
 
 // ntt.cu
 void build_twiddles(u64* d_tw, cudaStream_t st);
+bool ntt_columns_supported(unsigned logL, size_t cols);
+void ntt_columns(const u64* in, size_t rows, size_t cols, u64* out, unsigned logL, const u64* tw,
+                 cudaStream_t st);
 void ntt_batch(const u64* in, size_t in_stride, size_t n_in, u64* out, size_t out_stride,
                unsigned logN, size_t batch, u64* scratch, const u64* tw, cudaStream_t st);
 void transpose_u64(const u64* in, u64* out, size_t rows, size_t cols, size_t batch,
@@ -119,8 +122,13 @@ void eq_dot_dev(const void* vec, int is_bf, const ef2* point, unsigned k, ef2* o
 // a graph reads whichever buffer the slot names when it runs.
 void gemv_eq_rows(const u64* const* fref, const ef2* eq, size_t m, size_t n, ef2* out,
                   cudaStream_t st);
-void bits_gather(const u64* const* cwref, size_t two_n, const uint64_t* idx, unsigned s,
-                 size_t W, u64* bi, cudaStream_t st);
+struct EqTable {  // out[j] = eq(point[0 .. k), j)
+  const ef2* point;
+  unsigned k;
+  ef2* out;
+};
+void prove_prefix(const EqTable (&eqs)[3], const u64* const* cwref, size_t two_n,
+                  const uint64_t* idx, unsigned s, size_t W, u64* bi, cudaStream_t st);
 void g1_build(const u64* const* aref, size_t W, const ef2* eq_a2, unsigned C, ef2* g1,
               cudaStream_t st);
 void g2_build(const u64* bi, size_t W, unsigned s, const ef2* eq_r2, ef2* g2, cudaStream_t st);

@@ -33,15 +33,19 @@ void bf_commit(lgs_ctx* c, const u64* poly, int is_ef, size_t len, unsigned li,
   const size_t cols = ((size_t)1 << li) * (is_ef ? 2 : 1);
   const size_t L = rows << code_rate;
   const unsigned logL = ilog2(L);
-  u64* tT = ar.get<u64>(cols * rows);
-  u64* cT = ar.get<u64>(cols * L);
-  u64* scr = logL > 12 ? ar.get<u64>(cols * L) : nullptr;
-  transpose_u64(poly, tT, rows, cols, 1, st);
-  if (rs_dft_supported(logL, rows))  // cols <= 128
-    rs_dft_rows(tT, rows, rows, cT, L, logL, cols, scr, c->rs_tw.as<u64>(), st);
-  else
-    ntt_batch(tT, rows, rows, cT, L, logL, cols, scr, c->tw.as<u64>(), st);
-  transpose_u64(cT, out->codes, cols, L, 1, st);
+  if (ntt_columns_supported(logL, cols)) {
+    ntt_columns(poly, rows, cols, out->codes, logL, c->tw.as<u64>(), st);
+  } else {
+    u64* tT = ar.get<u64>(cols * rows);
+    u64* cT = ar.get<u64>(cols * L);
+    u64* scr = logL > 12 ? ar.get<u64>(cols * L) : nullptr;
+    transpose_u64(poly, tT, rows, cols, 1, st);
+    if (rs_dft_supported(logL, rows))  // cols <= 128
+      rs_dft_rows(tT, rows, rows, cT, L, logL, cols, scr, c->rs_tw.as<u64>(), st);
+    else
+      ntt_batch(tT, rows, rows, cT, L, logL, cols, scr, c->tw.as<u64>(), st);
+    transpose_u64(cT, out->codes, cols, L, 1, st);
+  }
   tl_mark("bf_dft_end", st);
   merkle_leaves_contig(out->codes, (unsigned)cols, L, out->nodes, st);
   tl_mark("bf_leaves_end", st);
@@ -941,10 +945,10 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
   // share a stream, so six chains run side by side: with ten, chains shared the hardware's work
   // queues and waited for one another by chance (prove alone, six against ten: 2^3 x 2^11 145 us
   // against 171, 2^6 x 2^14 240 against 276, 2^7 x 2^17 463 against 500, with the tiled sumchecks).
-  new_eq_dev(d_prm + P_z1, s.log_m, eqz1, st);
-  bits_gather(d_ptrs + PT_CW, two_n, d_idx, S, W, bi, st);
-  new_eq_dev(d_fields + fp.alpha2, 5, eq_a2, st);
-  new_eq_dev(d_fields + fp.r2, log_s, eq_r2, st);
+  prove_prefix({{d_prm + P_z1, s.log_m, eqz1},
+                {d_fields + fp.alpha2, 5, eq_a2},
+                {d_fields + fp.r2, log_s, eq_r2}},
+               d_ptrs + PT_CW, two_n, d_idx, S, W, bi, st);
   mark("prefix_end", st);
   LGS_CUDA(cudaEventRecord(c->ev_fork, st));
   std::vector<cudaStream_t> brs;
@@ -1042,15 +1046,19 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
   {
     t_tl_branch = "A2";
     cudaStream_t b = branch();
-    u64* t1 = ar.get<u64>(2 * n);
-    u64* t2 = ar.get<u64>(2 * two_n);
-    u64* scr = ilog2(two_n) > 12 ? ar.get<u64>(2 * two_n) : nullptr;
-    transpose_u64((const u64*)a_vec, t1, n, 2, 1, b);
-    if (rs_dft_supported(ilog2(two_n), n))
-      rs_dft_rows(t1, n, n, t2, two_n, ilog2(two_n), 2, scr, c->rs_tw.as<u64>(), b);
-    else
-      ntt_batch(t1, n, n, t2, two_n, ilog2(two_n), 2, scr, c->tw.as<u64>(), b);
-    transpose_u64(t2, (u64*)ra, 2, two_n, 1, b);
+    if (ntt_columns_supported(ilog2(two_n), 2)) {
+      ntt_columns((const u64*)a_vec, n, 2, (u64*)ra, ilog2(two_n), c->tw.as<u64>(), b);
+    } else {
+      u64* t1 = ar.get<u64>(2 * n);
+      u64* t2 = ar.get<u64>(2 * two_n);
+      u64* scr = ilog2(two_n) > 12 ? ar.get<u64>(2 * two_n) : nullptr;
+      transpose_u64((const u64*)a_vec, t1, n, 2, 1, b);
+      if (rs_dft_supported(ilog2(two_n), n))
+        rs_dft_rows(t1, n, n, t2, two_n, ilog2(two_n), 2, scr, c->rs_tw.as<u64>(), b);
+      else
+        ntt_batch(t1, n, n, t2, two_n, ilog2(two_n), 2, scr, c->tw.as<u64>(), b);
+      transpose_u64(t2, (u64*)ra, 2, two_n, 1, b);
+    }
     tl_mark("rs_end", b);
     y4_dev(eq_r2, ra, d_idx, S, (ef2*)(stage + S_y4), b);
     ef2* sel = ar.get<ef2>(two_n);
