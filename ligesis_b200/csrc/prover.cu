@@ -389,10 +389,13 @@ void commit_dev(lgs_ctx* c, const lgs_pk* pk, const u64* f, bool f_on_device,
     // the context stream, where the host-side staging of the next block is the slower part.
     StageTimer t(c->prof, c->st, "upload_and_rs_encode");
     // enough row blocks that the upload of each overlaps the encoding of the one before, but
-    // none smaller than upload_block (1 MB by default: a block costs a few calls and two
-    // launches, which a smaller block's overlap does not pay back; engine lanes use 4 MB, their
-    // jobs overlapping each other instead)
-    const size_t min_block = c->upload_block ? c->upload_block : ((size_t)1 << 20);
+    // none smaller than upload_block (by default 1 MB: a block costs a few calls and two
+    // launches, which a smaller block's overlap does not pay back; from 8 MB on 2 MB, which two
+    // host threads stage where one stages 1 MB, and four blocks are left: 2^6 x 2^14 opens in
+    // 0.92 instead of 1.04 ms, but 2^4 x 2^14, two blocks, in 0.62 instead of 0.54; engine lanes
+    // use 4 MB, their jobs overlapping each other instead)
+    const size_t min_block = c->upload_block ? c->upload_block
+                                             : (size_t)(m * n * 8 >= ((size_t)8 << 20) ? 2 : 1) << 20;
     unsigned nb = (unsigned)std::min<size_t>(lgs_ctx::ROW_BLOCKS, m);
     while (nb > 1 && m * n * 8 / nb < min_block) nb >>= 1;
     const size_t share = m / nb;  // m and nb are powers of two
