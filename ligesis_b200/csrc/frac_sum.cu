@@ -35,6 +35,7 @@
 #include <array>
 #include <cstring>
 
+#include "limb_sums.cuh"
 #include "prover.cuh"
 
 namespace lgs {
@@ -265,11 +266,12 @@ __device__ __forceinline__ void arr_store(ef2* out, size_t n, size_t e, const Q4
   st_ef(out + 3 * n + e, x.b1);
 }
 
-__device__ __forceinline__ void warp_sum3(ef2 (&s)[3]) {
-#pragma unroll
-  for (int q = 0; q < 3; ++q)
-#pragma unroll
-    for (int m = 16; m; m >>= 1) s[q] = ef_add(s[q], shfl_xor_ef(s[q], m));
+// Adds a warp's round sums to acc[3][6] (limb sums; the S(1) sums only where they are wanted).
+__device__ __forceinline__ void warp_add3(const ef2 (&s)[3], bool with_s1, uint32_t (*acc)[6],
+                                          unsigned lane) {
+  warp_add(s[0], acc[0], lane);
+  if (with_s1) warp_add(s[1], acc[1], lane);
+  warp_add(s[2], acc[2], lane);
 }
 
 __global__ void __launch_bounds__(FS_THREADS)
@@ -321,7 +323,10 @@ __global__ void __launch_bounds__(FS_THREADS)
   }
 }
 
-__global__ void __launch_bounds__(FS_THREADS, 2)
+// Three CTAs per SM (84 registers) and sums through limbs: at two the latency of the products and
+// loads showed, and adding field values across lanes was a fifth of the instructions (2^22 entries:
+// first pass 232 -> 204 us, the tails 54 -> 46).
+__global__ void __launch_bounds__(FS_THREADS, 3)
     fs_wide_kernel(const FsWide* __restrict__ jobs, unsigned njobs) {
   unsigned ji = 0;
   while (ji + 1 < njobs && blockIdx.x >= jobs[ji + 1].first_cta) ++ji;
@@ -329,15 +334,17 @@ __global__ void __launch_bounds__(FS_THREADS, 2)
   const bool ones = jb.in.ones != 0, s1f = jb.in.s1 != 0;
   const size_t g = (size_t)(blockIdx.x - jb.first_cta) * blockDim.x + threadIdx.x;
   const size_t nthr = jb.in.n >> jb.rounds;
+  __shared__ uint32_t red[2][3][6];  // limb sums of each round
+  if (threadIdx.x < 36) ((uint32_t*)red)[threadIdx.x] = 0;
   ef2 s0[3] = {ef_zero(), ef_zero(), ef_zero()};
   ef2 s1[3] = {ef_zero(), ef_zero(), ef_zero()};
   Q4 y;
   if (jb.rounds == 2) {
     const size_t e = g << 2;
     const Q4 x0 = arr_load(jb.in, e), x1 = arr_load(jb.in, e + 1);
-    const Q4 x2 = arr_load(jb.in, e + 2), x3 = arr_load(jb.in, e + 3);
     const unsigned j0 = (unsigned)(2 * g) & ((1u << FS_EQ_LO) - 1);
     const Q4 f0 = fs_pair(x0, x1, ld_ef(jb.lo[0] + j0), jb.c[0], ones, s1f, s0);
+    const Q4 x2 = arr_load(jb.in, e + 2), x3 = arr_load(jb.in, e + 3);
     const Q4 f1 = fs_pair(x2, x3, ld_ef(jb.lo[0] + j0 + 1), jb.c[0], ones, s1f, s0);
     y = fs_pair(f0, f1, ld_ef(jb.lo[1] + (g & ((1u << FS_EQ_LO) - 1))), jb.c[1], ones, s1f,
                 s1);
@@ -350,23 +357,15 @@ __global__ void __launch_bounds__(FS_THREADS, 2)
   arr_store(jb.fout, nthr, g, y, ones);
   // CTA sums of each round; round t's factor hi[j >> 10] is common to the CTA (256 threads cover
   // 512 or 256 consecutive pairs of an aligned block of 1024)
-  __shared__ ef2 red[2][3][8];
-  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  warp_sum3(s0);
-  if (jb.rounds == 2) warp_sum3(s1);
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      red[0][q][warp] = s0[q];
-      red[1][q][warp] = s1[q];
-    }
+  const unsigned lane = threadIdx.x & 31;
+  __syncthreads();  // red is clear
+  warp_add3(s0, s1f, red[0], lane);
+  if (jb.rounds == 2) warp_add3(s1, s1f, red[1], lane);
   __syncthreads();
   const size_t cta = blockIdx.x - jb.first_cta, ncta = nthr / FS_THREADS;
   if (threadIdx.x < 3 * jb.rounds) {
     const unsigned rd = threadIdx.x / 3, q = threadIdx.x % 3;
-    ef2 v = ef_zero();
-#pragma unroll
-    for (int w = 0; w < 8; ++w) v = ef_add(v, red[rd][q][w]);
+    const ef2 v = acc_value(red[rd][q]);
     const size_t g0 = cta * FS_THREADS;  // first thread of the CTA
     const size_t hj = rd == 0 ? (jb.rounds == 2 ? (g0 >> (FS_EQ_LO - 1)) : (g0 >> FS_EQ_LO))
                               : (g0 >> FS_EQ_LO);
@@ -378,19 +377,19 @@ __global__ void __launch_bounds__(FS_THREADS, 2)
 // Shared memory of a tail: weight tables (2^FS_TAIL_LOG entries), the folded elements after the
 // first round (2^(FS_TAIL_LOG-1)), per-warp round sums (FS_TAIL_LOG x 16 warps x 3).
 constexpr size_t FS_TAIL_SMEM = ((size_t)1 << FS_TAIL_LOG) * sizeof(ef2) +
-                                ((size_t)1 << (FS_TAIL_LOG - 1)) * sizeof(Q4) +
-                                (size_t)FS_TAIL_LOG * 16 * 3 * sizeof(ef2);
+                                ((size_t)1 << (FS_TAIL_LOG - 1)) * sizeof(Q4);
 constexpr unsigned FS_TAIL_THREADS = 512;  // latency-bound: as many warps as the registers allow
 
 __global__ void __launch_bounds__(FS_TAIL_THREADS) fs_tail_kernel(const FsTail* __restrict__ jobs) {
   extern __shared__ ef2 fs_sm[];
   ef2* wt = fs_sm;  // W_tau at offset 2^(nb - tau - 1) - 1
   Q4* xs = reinterpret_cast<Q4*>(fs_sm + (1u << FS_TAIL_LOG));
-  ef2* acc = fs_sm + (1u << FS_TAIL_LOG) + 4 * (1u << (FS_TAIL_LOG - 1));  // [tau][warp][3]
+  __shared__ uint32_t acc[FS_TAIL_LOG][3][6];  // limb sums of each round
   const FsTail& jb = jobs[blockIdx.x];
   const unsigned t0 = jb.t0, nb = jb.r - t0;
   const bool ones = jb.in.ones != 0, s1f = jb.in.s1 != 0;
-  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (unsigned i = threadIdx.x; i < FS_TAIL_LOG * 18; i += blockDim.x) ((uint32_t*)acc)[i] = 0;
 
   // W_{nb-1} = [1]; W_tau[2m + b] = W_{tau+1}[m] eq(z_{t0+tau+1}, b): the weight of pair jl in
   // round t0+tau is E_{t0+tau+1}(jl).
@@ -404,12 +403,6 @@ __global__ void __launch_bounds__(FS_TAIL_THREADS) fs_tail_kernel(const FsTail* 
   }
   __syncthreads();
 
-  auto warp_acc = [&](ef2 (&s)[3], unsigned tau) {  // per-warp sums, no block barrier
-    warp_sum3(s);
-    if (lane == 0)
-#pragma unroll
-      for (int q = 0; q < 3; ++q) acc[(tau * nw + warp) * 3 + q] = s[q];
-  };
   {  // round t0 from global memory
     const unsigned np = 1u << (nb - 1);
     const ef2 c = ld_ef(jb.ch + t0);
@@ -418,7 +411,7 @@ __global__ void __launch_bounds__(FS_TAIL_THREADS) fs_tail_kernel(const FsTail* 
       const Q4 lo = arr_load(jb.in, 2 * jl), hi = arr_load(jb.in, 2 * jl + 1);
       xs[jl] = fs_pair(lo, hi, wt[np - 1 + jl], c, ones, s1f, s);
     }
-    warp_acc(s, 0);
+    warp_add3(s, s1f, acc[0], lane);
   }
   // rounds with more pairs than one warp: exchange through shared memory with barriers
   unsigned tau = 1;
@@ -440,31 +433,24 @@ __global__ void __launch_bounds__(FS_TAIL_THREADS) fs_tail_kernel(const FsTail* 
       const unsigned jl = threadIdx.x + q * blockDim.x;
       if (jl < np) xs[jl] = o[q];
     }
-    warp_acc(s, tau);
+    warp_add3(s, s1f, acc[tau], lane);
   }
   __syncthreads();
-  // the rest in warp 0 (the other warps' sums of these rounds are zero)
-  for (; tau < nb; ++tau) {
+  for (; warp == 0 && tau < nb; ++tau) {  // the rest in warp 0
     const unsigned np = 1u << (nb - tau - 1);
     ef2 s[3] = {ef_zero(), ef_zero(), ef_zero()};
-    if (warp == 0) {
-      const ef2 c = ld_ef(jb.ch + t0 + tau);
-      Q4 o;
-      if (lane < np)
-        o = fs_pair(xs[2 * lane], xs[2 * lane + 1], wt[np - 1 + lane], c, ones, s1f, s);
-      __syncwarp();
-      if (lane < np) xs[lane] = o;
-      __syncwarp();
-    }
-    warp_acc(s, tau);
+    const ef2 c = ld_ef(jb.ch + t0 + tau);
+    Q4 o;
+    if (lane < np)
+      o = fs_pair(xs[2 * lane], xs[2 * lane + 1], wt[np - 1 + lane], c, ones, s1f, s);
+    __syncwarp();
+    if (lane < np) xs[lane] = o;
+    __syncwarp();
+    warp_add3(s, s1f, acc[tau], lane);
   }
   __syncthreads();
-  for (unsigned i = threadIdx.x; i < nb * 3; i += blockDim.x) {
-    const unsigned tt = i / 3, q = i % 3;
-    ef2 v = ef_zero();
-    for (unsigned w = 0; w < nw; ++w) v = ef_add(v, acc[(tt * nw + w) * 3 + q]);
-    st_ef(jb.part + i, v);
-  }
+  for (unsigned i = threadIdx.x; i < nb * 3; i += blockDim.x)
+    st_ef(jb.part + i, acc_value(acc[i / 3][i % 3]));
   if (threadIdx.x == 0) {
     const Q4 x = xs[0];
     st_ef(jb.leaves + 0, x.a0);
@@ -476,25 +462,17 @@ __global__ void __launch_bounds__(FS_TAIL_THREADS) fs_tail_kernel(const FsTail* 
 
 // Sums the partial sums of each round: one CTA per round.
 __global__ void __launch_bounds__(FS_THREADS) fs_sums_kernel(const FsRound* __restrict__ rounds) {
-  __shared__ ef2 red[96];
+  __shared__ uint32_t acc[3][6];
+  if (threadIdx.x < 18) ((uint32_t*)acc)[threadIdx.x] = 0;
   const FsRound& rd = rounds[blockIdx.x];
   ef2 s[3] = {ef_zero(), ef_zero(), ef_zero()};
   for (unsigned i = threadIdx.x; i < rd.ncta; i += blockDim.x)
 #pragma unroll
     for (int q = 0; q < 3; ++q) s[q] = ef_add(s[q], ld_ef(rd.part + (size_t)i * 3 + q));
-  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  warp_sum3(s);
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < 3; ++q) red[q * 32 + warp] = s[q];
   __syncthreads();
-  if (warp != 0) return;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) s[q] = lane < nw ? red[q * 32 + lane] : ef_zero();
-  warp_sum3(s);
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < 3; ++q) st_ef(rd.out + q, s[q]);
+  warp_add3(s, true, acc, threadIdx.x & 31);
+  __syncthreads();
+  if (threadIdx.x < 3) st_ef(rd.out + threadIdx.x, acc_value(acc[threadIdx.x]));
 }
 
 // g(x) = K(x) S(x) with S quadratic: S(2) = -S(0) + 2 S(1) + 2 L, S(3) = -2 S(0) + 3 S(1) + 6 L
