@@ -74,6 +74,7 @@ constexpr int NBARS = 3 * TC_STAGES + 2 * W_STAGES + 5;
 constexpr int SMEM_BYTES =
     TC_STAGES * STAGE_BYTES + W_STAGES * W_BYTES + 1024 /*align*/ + 512 /*barriers*/;
 static_assert(NBARS * 8 + 4 <= 512, "barrier space");
+static_assert(TC_SUB == 2, "the MMA loop issues a stage's two chunks");
 constexpr long long WAIT_CYCLES = tc::DRAIN_CYCLES;  // ~2 s at 1.9 GHz (default budget)
 constexpr uint32_t IDESC_PAIR = tc::idesc_u8(256, 256);
 constexpr uint32_t IDESC = tc::idesc_u8(128, 256);  // the peak microbenchmark's MMA
