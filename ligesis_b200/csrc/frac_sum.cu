@@ -3,8 +3,8 @@
 //
 // The circuit is a binary tree of fraction additions over 2^k inputs: level s-1 pairs level s
 // along the low bit, p' = p0 q1 + p1 q0, q' = q0 q1.  Every level is kept (level s at offset
-// 2^s - 1 of the P and Q arrays); a launch of fs_build_kernel computes up to FS_BUILD_T levels of
-// one subtree per CTA in shared memory.
+// 2^s - 1 of the P and Q arrays); a launch of fs_build_kernel computes up to FS_BUILD_T levels
+// per CTA in shared memory.
 //
 // Layer r (r = 0 .. k-1) proves the claim on level r at the point z_r with a degree-3 sumcheck
 // over r rounds on the low-bit splits A0, A1, B0, B1 of level r+1, binding the low bit first.
@@ -43,7 +43,8 @@ namespace lgs {
 namespace {
 
 constexpr unsigned FS_THREADS = 256;
-constexpr unsigned FS_BUILD_T = 10;  // tree levels per build launch
+constexpr unsigned FS_BUILD_T = 10;     // tree levels per build launch of few CTAs
+constexpr unsigned FS_BUILD_SHORT = 5;  // and of 512 or more
 constexpr unsigned FS_MAX_K = 28;
 
 __device__ __forceinline__ ef2 ld_ef(const ef2* p) {
@@ -79,16 +80,20 @@ __device__ __forceinline__ ef2 src_q(const FsSrc& s, size_t i) {
   return s.q_sub ? ef_sub(s.alpha, v) : v;
 }
 
-// Levels S-1 .. S-T of the tree from level S: CTA c reduces entries [c 2^T, (c+1) 2^T) of level
-// S (frac_sum.rs:124-136).  Shared memory: a chain of the levels, p then q (2 x 2^T entries).
+// Levels S-1 .. S-T of the tree from level S: CTA c reduces entries [c 2^E, (c+1) 2^E) of level
+// S, E >= T (frac_sum.rs:124-136).  Shared memory: a chain of the levels, p then q (2 x 2^E entries).
+// A level halves the threads at work, so a launch over many CTAs stops at T = 5 of E = 10, where
+// most of its warps would only wait (2^22 entries: 69 -> 53 us, and 3 more in the launches after;
+// with 64 or 128 CTAs the extra launch costs what it saves).
 __global__ void __launch_bounds__(FS_THREADS)
-    fs_build_kernel(FsSrc src, unsigned S, unsigned T, ef2* __restrict__ P, ef2* __restrict__ Q) {
+    fs_build_kernel(FsSrc src, unsigned S, unsigned E, unsigned T, ef2* __restrict__ P,
+                    ef2* __restrict__ Q) {
   extern __shared__ ef2 fs_sm[];
   ef2* sp = fs_sm;
-  ef2* sq = fs_sm + ((size_t)1 << T);
-  const unsigned half = 1u << (T - 1);
-  const size_t base = (size_t)blockIdx.x << T;
-  size_t gout = (((size_t)1 << (S - 1)) - 1) + ((size_t)blockIdx.x << (T - 1));
+  ef2* sq = fs_sm + ((size_t)1 << E);
+  const unsigned half = 1u << (E - 1);
+  const size_t base = (size_t)blockIdx.x << E;
+  size_t gout = (((size_t)1 << (S - 1)) - 1) + ((size_t)blockIdx.x << (E - 1));
   for (unsigned i = threadIdx.x; i < half; i += blockDim.x) {
     const size_t e = base + 2 * i;
     const ef2 q0 = src_q(src, e), q1 = src_q(src, e + 1);
@@ -107,7 +112,7 @@ __global__ void __launch_bounds__(FS_THREADS)
   for (unsigned l = 2; l <= T; ++l) {
     __syncthreads();
     const unsigned nc = cnt >> 1;
-    gout = (((size_t)1 << (S - l)) - 1) + ((size_t)blockIdx.x << (T - l));
+    gout = (((size_t)1 << (S - l)) - 1) + ((size_t)blockIdx.x << (E - l));
     for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) {
       const ef2 p0 = sp[off + 2 * i], p1 = sp[off + 2 * i + 1];
       const ef2 q0 = sq[off + 2 * i], q1 = sq[off + 2 * i + 1];
@@ -830,9 +835,10 @@ static void fs_launch(const FsPlan& pl, uint8_t* pinned, cudaStream_t st) {
     unsigned S = k;
     FsSrc src = pl.in;
     while (S > 0) {
-      const unsigned T = std::min(S, FS_BUILD_T);
-      const size_t smem = 2 * ((size_t)1 << T) * sizeof(ef2);
-      fs_build_kernel<<<(unsigned)((size_t)1 << (S - T)), FS_THREADS, smem, st>>>(src, S, T, P, Q);
+      const unsigned E = std::min(S, FS_BUILD_T), T = S >= E + 9 ? FS_BUILD_SHORT : E;
+      const size_t smem = 2 * ((size_t)1 << E) * sizeof(ef2);
+      fs_build_kernel<<<(unsigned)((size_t)1 << (S - E)), FS_THREADS, smem, st>>>(src, S, E, T, P,
+                                                                                  Q);
       LGS_LAUNCH_CHECK();
       S -= T;
       src = FsSrc{P + ((size_t)1 << S) - 1, Q + ((size_t)1 << S) - 1, ef_zero(), 0};
