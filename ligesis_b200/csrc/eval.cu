@@ -544,29 +544,47 @@ void sel_build(const uint64_t* idx, const ef2* eq_r2, unsigned s, size_t two_n, 
   sel_scatter_kernel<<<cdiv(s, 128), 128, 0, st>>>(idx, eq_r2, s, sel);
   LGS_LAUNCH_CHECK();
 }
-// w[k] = prod_t (1 - r3[t] + r3[t] g^((2^t k) mod 2n)) (pcs/src/ligesis.rs:553-567)
-__global__ void rs_weights_kernel(const ef2* __restrict__ r3, unsigned log2n, size_t n,
-                                  const u64* __restrict__ tw, ef2* __restrict__ w) {
-  __shared__ ef2 r[64];
-  if (threadIdx.x < log2n) r[threadIdx.x] = r3[threadIdx.x];
+// w[k] = prod_t (1 - r3[t] + r3[t] g^((2^t k) mod 2n)) (pcs/src/ligesis.rs:553-567).  The factors
+// of t >= t1 depend on the low log2n - t1 bits of k alone: tab[k & tab_mask] holds their product.
+__global__ void rs_weights_kernel(const ef2* __restrict__ r3, unsigned log2n, unsigned t0,
+                                  unsigned t1, size_t n, const u64* __restrict__ tw,
+                                  const ef2* __restrict__ tab, size_t tab_mask,
+                                  ef2* __restrict__ w) {
+  __shared__ ef2 r[64], omr[64];
+  if (threadIdx.x < log2n) {
+    r[threadIdx.x] = r3[threadIdx.x];
+    omr[threadIdx.x] = ef_sub(ef_one(), r3[threadIdx.x]);
+  }
   __syncthreads();
   size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const size_t mask = ((size_t)2 << (log2n - 1)) - 1;
   const unsigned shift = TW_LOG - log2n;
-  ef2 prod = ef_one();
-  for (unsigned t = 0; t < log2n; ++t) {
+  ef2 prod = tab ? tab[k & tab_mask] : ef_one();
+  for (unsigned t = t0; t < t1; ++t) {
     size_t e = (k << t) & mask;
     u64 gp = __ldg(tw + (e << shift));
-    ef2 term = ef_add(ef_sub(ef_one(), r[t]), ef_scale(r[t], gp));
-    prod = ef_mul(prod, term);
+    prod = ef_mul(prod, ef_add(omr[t], ef_scale(r[t], gp)));
   }
   w[k] = prod;
 }
-void rs_weights_dev(const ef2* r3, unsigned log2n, size_t n, const u64* tw, ef2* w,
+// From 2^17 weights on the last 12 factors come from a table made first: 2^17
+// weights 26 -> 20 us in two launches.  Below, one launch is mostly latency and a second adds to
+// it (2^7 x 2^16 opens in 848 us with two, 843 with one).  scratch: 2^12 values.
+void rs_weights_dev(const ef2* r3, unsigned log2n, size_t n, const u64* tw, ef2* w, ef2* scratch,
                     cudaStream_t st) {
   if (log2n > TW_LOG || log2n > 64) throw ShapeError("rs_weights: domain too large");
-  rs_weights_kernel<<<cdiv(n, 256), 256, 0, st>>>(r3, log2n, n, tw, w);
+  constexpr unsigned TAB = 12;
+  const bool split = log2n >= 18;
+  const unsigned t1 = split ? log2n - TAB : log2n;
+  if (split) {
+    rs_weights_kernel<<<(1u << TAB) / 128, 128, 0, st>>>(r3, log2n, t1, log2n, (size_t)1 << TAB,
+                                                         tw, nullptr, 0, scratch);
+    LGS_LAUNCH_CHECK();
+  }
+  rs_weights_kernel<<<cdiv(n, 256), 256, 0, st>>>(r3, log2n, 0, t1, n, tw,
+                                                  split ? scratch : nullptr,
+                                                  ((size_t)1 << TAB) - 1, w);
   LGS_LAUNCH_CHECK();
 }
 

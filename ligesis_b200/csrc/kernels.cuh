@@ -137,7 +137,7 @@ void y4_dev(const ef2* eq_r2, const ef2* ra, const uint64_t* idx, unsigned s, ef
             cudaStream_t st);
 void sel_build(const uint64_t* idx, const ef2* eq_r2, unsigned s, size_t two_n, ef2* sel,
                cudaStream_t st);
-void rs_weights_dev(const ef2* r3, unsigned log2n, size_t n, const u64* tw, ef2* w,
+void rs_weights_dev(const ef2* r3, unsigned log2n, size_t n, const u64* tw, ef2* w, ef2* scratch,
                     cudaStream_t st);
 // Basefold batched-open helpers.
 struct BfChannelDev {

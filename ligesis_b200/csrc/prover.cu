@@ -1081,7 +1081,7 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
     cudaStream_t b = branch();
     ef2* w = ar.get<ef2>(n);
     ef2* ga = ar.get<ef2>(n);
-    rs_weights_dev(d_prm + P_r3, log_n + 1, n, c->tw.as<u64>(), w, b);
+    rs_weights_dev(d_prm + P_r3, log_n + 1, n, c->tw.as<u64>(), w, ga, b);  // ga is written next
     combine_eq_dev(d_prm + P_apts, 2, log_n, d_fields + fp.gamma_a, ga, b);
     ScJob j[2] = {};
     j[0].src[1] = j[0].dst[1] = w;
