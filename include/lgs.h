@@ -289,8 +289,8 @@ lgs_status lgs_profile_names(lgs_ctx* ctx, char* buf, size_t cap, size_t* needed
  *                      fits 24 and every weight 16 signed bits (else the CUDA cores), 1 always
  *                      the CUDA cores
  *   "upload_block_bytes" commits of host polynomials: the least bytes per row block of the
- *                      upload pipelined with the RS encoding (0: 1 MB, from 8 MB on 2; an engine's lanes
- *                      start at 4 MB)
+ *                      upload pipelined with the RS encoding (0: 4 MB, 8 MB if pageable; an
+ *                      engine's lanes start at 4 MB)
  *   "upload_tail_rows" commits of host polynomials: rows of the last of those row blocks, whose
  *                      RS encoding the prove waits for after the upload (0, or a whole equal
  *                      share or more: equal blocks)

@@ -10,6 +10,10 @@
 #include <mutex>
 #include <thread>
 
+#if defined(__x86_64__)
+#include <emmintrin.h>
+#endif
+
 #include "prover.cuh"
 
 namespace lgs {
@@ -57,6 +61,35 @@ void bf_commit(lgs_ctx* c, const u64* poly, int is_ef, size_t len, unsigned li,
   out->L = L;
 }
 
+// Copy into page-locked memory that the DMA engine reads next.  Its reads of lines that a core
+// still holds modified come back one snoop at a time: 8 MB just written by eight threads moved at 8
+// GB/s, and at 51 once written past the caches.
+void stage_copy(void* dst, const void* src, size_t bytes) {
+#if defined(__x86_64__)
+  char* d = (char*)dst;
+  const char* p = (const char*)src;
+  const size_t head = std::min(bytes, (size_t)(-(uintptr_t)d & 63));
+  std::memcpy(d, p, head);
+  size_t i = head;
+  for (; i + 64 <= bytes; i += 64) {
+    const __m128i v0 = _mm_loadu_si128((const __m128i*)(p + i));
+    const __m128i v1 = _mm_loadu_si128((const __m128i*)(p + i + 16));
+    const __m128i v2 = _mm_loadu_si128((const __m128i*)(p + i + 32));
+    const __m128i v3 = _mm_loadu_si128((const __m128i*)(p + i + 48));
+    _mm_stream_si128((__m128i*)(d + i), v0);
+    _mm_stream_si128((__m128i*)(d + i + 16), v1);
+    _mm_stream_si128((__m128i*)(d + i + 32), v2);
+    _mm_stream_si128((__m128i*)(d + i + 48), v3);
+  }
+  std::memcpy(d + i, p + i, bytes - i);
+  _mm_sfence();
+#else
+  std::memcpy(dst, src, bytes);
+#endif
+}
+
+void plain_copy(void* dst, const void* src, size_t bytes) { std::memcpy(dst, src, bytes); }
+
 // Host threads shared by every context of the process for large pageable-to-pinned copies: one
 // thread's memcpy reaches a fraction of the host's memory bandwidth.
 class CopyPool {
@@ -65,11 +98,12 @@ class CopyPool {
     static CopyPool* pool = new CopyPool;  // never destroyed: its threads wait until exit
     return *pool;
   }
-  // memcpy split into parts of at least 1 MiB, run by the pool's threads and the caller.
-  void copy(void* dst, const void* src, size_t bytes) {
+  using Copy = void (*)(void*, const void*, size_t);
+  // A copy split into parts of at least 1 MiB, run by the pool's threads and the caller.
+  void copy(void* dst, const void* src, size_t bytes, Copy fn) {
     const size_t parts = std::min<size_t>(threads_.size() + 1, std::max<size_t>(1, bytes >> 20));
     if (parts <= 1) {
-      std::memcpy(dst, src, bytes);
+      fn(dst, src, bytes);
       return;
     }
     const size_t step = (bytes / parts + 63) & ~(size_t)63;
@@ -81,12 +115,12 @@ class CopyPool {
         const size_t len = std::min(bytes, off + step) - off;
         if (len) {
           ++batch.left;
-          tasks_.push_back({(char*)dst + off, (const char*)src + off, len, &batch});
+          tasks_.push_back({(char*)dst + off, (const char*)src + off, len, fn, &batch});
         }
       }
     }
     cv_.notify_all();
-    std::memcpy(dst, src, std::min(bytes, step));
+    fn(dst, src, std::min(bytes, step));
     std::unique_lock<std::mutex> lk(mu_);
     batch.cv.wait(lk, [&] { return batch.left == 0; });
   }
@@ -100,6 +134,7 @@ class CopyPool {
     char* dst;
     const char* src;
     size_t len;
+    Copy fn;
     Batch* batch;
   };
   CopyPool() {
@@ -116,7 +151,7 @@ class CopyPool {
       Task t = tasks_.front();
       tasks_.pop_front();
       lk.unlock();
-      std::memcpy(t.dst, t.src, t.len);
+      t.fn(t.dst, t.src, t.len);
       lk.lock();
       if (--t.batch->left == 0) t.batch->cv.notify_all();
     }
@@ -152,9 +187,9 @@ void h2d_staged(lgs_ctx* c, void* dst, const void* src, size_t bytes, cudaStream
     LGS_CUDA(cudaEventSynchronize(c->ring_ev[slot]));  // the slot's previous copy has landed
     c->ring[slot].reserve(lgs_ctx::RING_CHUNK);
     if (c->copy_pool)
-      CopyPool::get().copy(c->ring[slot].p, (const char*)src + off, len);
+      CopyPool::get().copy(c->ring[slot].p, (const char*)src + off, len, stage_copy);
     else
-      std::memcpy(c->ring[slot].p, (const char*)src + off, len);
+      stage_copy(c->ring[slot].p, (const char*)src + off, len);
     LGS_CUDA(cudaMemcpyAsync((char*)dst + off, c->ring[slot].p, len, cudaMemcpyHostToDevice, st));
     LGS_CUDA(cudaEventRecord(c->ring_ev[slot], st));
   }
@@ -168,7 +203,7 @@ void d2h_staged(lgs_ctx* c, void* dst, const void* src, size_t bytes, cudaStream
     const size_t len = std::min(CHUNK, bytes - off);
     LGS_CUDA(cudaEventSynchronize(c->ring_ev[slot]));
     if (c->copy_pool)
-      CopyPool::get().copy((char*)dst + off, c->ring[slot].p, len);
+      CopyPool::get().copy((char*)dst + off, c->ring[slot].p, len, plain_copy);
     else
       std::memcpy((char*)dst + off, c->ring[slot].p, len);
   };
@@ -389,13 +424,15 @@ void commit_dev(lgs_ctx* c, const lgs_pk* pk, const u64* f, bool f_on_device,
     // the context stream, where the host-side staging of the next block is the slower part.
     StageTimer t(c->prof, c->st, "upload_and_rs_encode");
     // enough row blocks that the upload of each overlaps the encoding of the one before, but
-    // none smaller than upload_block (by default 1 MB: a block costs a few calls and two
-    // launches, which a smaller block's overlap does not pay back; from 8 MB on 2 MB, which two
-    // host threads stage where one stages 1 MB, and four blocks are left: 2^6 x 2^14 opens in
-    // 0.92 instead of 1.04 ms, but 2^4 x 2^14, two blocks, in 0.62 instead of 0.54; engine lanes
-    // use 4 MB, their jobs overlapping each other instead)
-    const size_t min_block = c->upload_block ? c->upload_block
-                                             : (size_t)(m * n * 8 >= ((size_t)8 << 20) ? 2 : 1) << 20;
+    // none smaller than upload_block: a block costs a few calls and two launches, which a smaller
+    // block's overlap does not pay back.  Page-locked f: 4 MB by default (2^5 x 2^14 opens in 438 us
+    // as one block, 466 as four of 1 MB; from 2^6 x 2^15 on within 1 %).  Pageable f: 8 MB, a 1
+    // MB part for each of the pool's threads; smaller blocks are staged by fewer, and the staging
+    // is the slower part (2^6 x 2^14 in 0.66 ms as one block, 0.72 as two, 0.99 as eight; 2^6 x
+    // 2^15 in 0.93 as two or four, 1.08 as eight).  Engine lanes use 4 MB, their jobs overlapping
+    // each other instead.
+    const bool pinned = host_is_pinned(f);
+    const size_t min_block = c->upload_block ? c->upload_block : (size_t)(pinned ? 4 : 8) << 20;
     unsigned nb = (unsigned)std::min<size_t>(lgs_ctx::ROW_BLOCKS, m);
     while (nb > 1 && m * n * 8 / nb < min_block) nb >>= 1;
     const size_t share = m / nb;  // m and nb are powers of two
@@ -414,7 +451,6 @@ void commit_dev(lgs_ctx* c, const lgs_pk* pk, const u64* f, bool f_on_device,
       for (unsigned b = 0; b + 1 < nb; ++b) brow[b + 1] = (size_t)(b + 1) * share;
     }
     brow[nb] = m;
-    const bool pinned = host_is_pinned(f);
     cudaStream_t cp = c->side[0];
     if (pinned) {
       LGS_CUDA(cudaEventRecord(c->ev_fork, c->st));  // cd->f exists on the context stream
@@ -872,7 +908,7 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
   const ef2* d_fields = d_prm + P_fields;
   const uint64_t* d_idx = (const uint64_t*)(d_up + U_idx);
   const ef2* pts[3] = {d_prm + P_pa, d_prm + P_rbi, d_prm + P_ra};
-  std::memcpy(h_up + U_prm, prm.data(), prm.size() * sizeof(ef2));
+  stage_copy(h_up + U_prm, prm.data(), prm.size() * sizeof(ef2));
   std::memcpy(h_up + U_idx, idx.data(), S * 8);
   const u64* const* d_ptrs = (const u64* const*)(d_up + U_ptrs);
   {
@@ -897,7 +933,7 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
       chs[ch].li = chan_li[ch];
       chs[ch].point = pts[ch];
     }
-    std::memcpy(h_up + U_gidx, plan.idx.data(), plan.idx.size() * 8);
+    stage_copy(h_up + U_gidx, plan.idx.data(), plan.idx.size() * 8);
     GatherSeg* segs = (GatherSeg*)(h_up + U_segs);
     for (size_t i = 0; i < plan.segs.size(); ++i) {
       segs[i] = plan.segs[i];
@@ -1372,7 +1408,7 @@ void basefold_prove_dev(lgs_ctx* c, const lgs_basefold* bf, const u64* point_hos
     ch->point = d_pt;
     const u64* pp = bf->poly.as<u64>();
     std::memcpy(h_up + U_ptr, &pp, sizeof(pp));
-    std::memcpy(h_up + U_gidx, plan.idx.data(), plan.idx.size() * 8);
+    stage_copy(h_up + U_gidx, plan.idx.data(), plan.idx.size() * 8);
     GatherSeg* segs = (GatherSeg*)(h_up + U_segs);
     for (size_t i = 0; i < plan.segs.size(); ++i) {
       segs[i] = plan.segs[i];
