@@ -679,6 +679,11 @@ bool block_witness_dev(lgs_ctx* c, const int64_t* x, unsigned n, unsigned d, uns
       !gelu_len || scale <= 0 || score_scale <= 0 || n > 65536 || d > (1u << 22) ||
       hidden > (1u << 24) || (size_t)heads * n > ((size_t)1 << 24))
     return false;
+  // All weights and results are resident at once here and one layer's at a time there, so blocks of
+  // gigabytes (GPT-2's is 0.1) keep to the layers.
+  const double words = 4.0 * d * d + 2.0 * d * hidden + n * (20.0 * d + 4.0 * hidden) +
+                       5.0 * heads * n * (double)n + (double)exp_len + (double)gelu_len;
+  if (words > (double)((size_t)1 << 29)) return false;  // 4 GB
   cudaStream_t st = c->st;
   Arena& ar = c->arena;
   ar.begin();
