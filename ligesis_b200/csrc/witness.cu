@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(256, 2) linear_witness_kernel(const LwArgs a) 
       else
         a.part[(size_t)blockIdx.z * a.rows * a.cols + o] = acc[i][j];
     }
-  if (bad) set_err(a.err);
+  if (bad) set_flag(a.err);
 }
 
 // Sums the K splits of every output (exactly) and finishes it.
@@ -255,7 +255,7 @@ __global__ void linear_witness_finish_kernel(const LwArgs a, unsigned nsplit) {
     for (unsigned z = 0; z < nsplit; ++z) add128(s, a.part[(size_t)z * n + o]);
     bad |= !lw_finish(s, a.bias, o % a.cols, a.d, o, a.q, a.rem, a.y, a.yf);
   }
-  if (bad) set_err(a.err);
+  if (bad) set_flag(a.err);
 }
 
 // layer_norm (proofsys/src/model.rs:241-279), one CTA per row: exact 128-bit sums of x and x^2,
@@ -337,6 +337,12 @@ __global__ void __launch_bounds__(256) layer_norm_witness_kernel(const LnArgs a)
   if (bad) atomicOr(a.err, 1);
 }
 
+void throw_if_timed_out(const int* flags) {
+  if (flags[LW_WAIT])
+    throw DeviceTimeout("linear witness: a bounded device wait gave up (code " +
+                        std::to_string(flags[LW_WAIT]) + ")");
+}
+
 }  // namespace
 
 void linear_witness_dev(lgs_ctx* c, const int64_t* x, size_t rows, size_t inner, const int64_t* w,
@@ -368,31 +374,27 @@ void linear_witness_dev(lgs_ctx* c, const int64_t* x, size_t rows, size_t inner,
     dy = ar.get<int64_t>(no);
     df = y_field ? ar.get<uint64_t>(no) : nullptr;
   }
-  // Error word, then the tensor path's operand-range flag, in pinned memory that the kernels reach:
-  // they write it only when something is wrong, so a call needs no memset and no copy for it, and
-  // its one wait is the stream's (vocabulary head 119 -> 108 us a call, 1 x 32 x 32: 84 -> 67).
+  // The layer's flags (LwFlag), in pinned memory that the kernels reach: they write it only when
+  // something is wrong, so a call needs no memset and no copy for it, and its one wait is the
+  // stream's (vocabulary head 119 -> 108 us a call, 1 x 32 x 32: 84 -> 67).
   if (!c->wit_flags.p) {
-    c->wit_flags.reserve(2 * sizeof(int));
-    std::memset(c->wit_flags.p, 0, 2 * sizeof(int));
+    c->wit_flags.reserve(LW_FLAGS * sizeof(int));
+    std::memset(c->wit_flags.p, 0, LW_FLAGS * sizeof(int));
   }
-  int* derr = c->wit_flags.as<int>();
-  int flags[2];
+  int* dflags = c->wit_flags.as<int>();
+  int flags[LW_FLAGS];
   auto read_flags = [&] {
     LGS_CUDA(cudaStreamSynchronize(st));
-    for (int i = 0; i < 2; ++i) flags[i] = ((volatile int*)derr)[i], derr[i] = 0;
+    for (int i = 0; i < LW_FLAGS; ++i) flags[i] = ((volatile int*)dflags)[i], dflags[i] = 0;
   };
-  int herr = 0;
   bool done = false;
   if (c->witness_path == 0) {
     // operands within the limb encodings (every integer GPT-2 layer): the tensor cores
     linear_witness_tc(c, dx, rows, inner, dw, cols, w_transposed, db, divisor, dq, dr, dy, df,
-                      derr, derr + 1);
+                      dflags);
     read_flags();
-    if (flags[0] >= 16)
-      throw DeviceTimeout("linear witness: a bounded device wait gave up (code " +
-                          std::to_string(flags[0]) + ")");
-    done = flags[1] == 0;  // else an operand needs more than its limbs: the CUDA-core kernel
-    if (done) herr = flags[0];
+    throw_if_timed_out(flags);
+    done = !flags[LW_OPERAND];  // else an operand needs more than its limbs: the CUDA-core kernel
   }
   if (!done) {
   // Few rows (GPT-2 runs 31 positions) leave most SMs idle: split K until there are about two
@@ -407,7 +409,7 @@ void linear_witness_dev(lgs_ctx* c, const int64_t* x, size_t rows, size_t inner,
   kchunk = (kchunk + LW_K - 1) / LW_K * LW_K;
   split = (inner + kchunk - 1) / kchunk;
   LwArgs a{dx, dw, db, rows, inner, cols, kchunk, divisor, w_transposed ? 1 : 0, nullptr,
-           dq, dr, dy, df, derr};
+           dq, dr, dy, df, dflags + LW_RESULT};
   const dim3 grid((unsigned)((cols + LW_TN - 1) / LW_TN), (unsigned)((rows + LW_TM - 1) / LW_TM),
                   (unsigned)split);
   LGS_CUDA(cudaFuncSetAttribute(linear_witness_kernel<true>,
@@ -427,7 +429,6 @@ void linear_witness_dev(lgs_ctx* c, const int64_t* x, size_t rows, size_t inner,
     LGS_LAUNCH_CHECK();
   }
   read_flags();
-  herr = flags[0];
   }
   if (!on_device) {
     LGS_CUDA(cudaMemcpyAsync(q, dq, no * 8, cudaMemcpyDeviceToHost, st));
@@ -436,7 +437,8 @@ void linear_witness_dev(lgs_ctx* c, const int64_t* x, size_t rows, size_t inner,
     if (y_field) LGS_CUDA(cudaMemcpyAsync(y_field, df, no * 8, cudaMemcpyDeviceToHost, st));
     LGS_CUDA(cudaStreamSynchronize(st));
   }
-  if (herr) throw ShapeError("linear witness: a product or Q + bias leaves the i64 range");
+  if (flags[LW_RESULT])
+    throw ShapeError("linear witness: a product or Q + bias leaves the i64 range");
 }
 
 }  // namespace lgs
@@ -700,7 +702,7 @@ bool block_witness_dev(lgs_ctx* c, const int64_t* x, unsigned n, unsigned d, uns
   for (int i = 0; i < 36; ++i) off[i + 1] = off[i] + (size[i] + 31) / 32 * 32;
   int64_t* o = ar.get<int64_t>(off[36]);
   auto fld = [&](int i) { return o + off[i]; };
-  constexpr int NERR = 16;  // two words per linear layer (8), then one per other step
+  constexpr int NLIN = 4 * LW_FLAGS, NERR = NLIN + 6;  // four linear layers, then the other steps
   int* derr = ar.get<int>(NERR);
   LGS_CUDA(cudaMemsetAsync(derr, 0, NERR * sizeof(int), st));
   // Uploads go on a stream of their own, so that a ring slot is free as soon as its copy is done
@@ -735,10 +737,10 @@ bool block_witness_dev(lgs_ctx* c, const int64_t* x, unsigned n, unsigned d, uns
     LGS_LAUNCH_CHECK();
   };
   auto linear = [&](const int64_t* xin, size_t inner, const int64_t* wt, int b, size_t cols,
-                    int64_t* q, int64_t* rem, int64_t* y, int* err) {
+                    int64_t* q, int64_t* rem, int64_t* y, int* flags) {
     const int64_t* dw = in(wt, inner * cols);
     linear_witness_tc(c, xin, n, inner, dw, cols, false, dv + at[b], scale, q, rem, y, nullptr,
-                      err, err + 1);
+                      flags);
   };
   auto add = [&](const int64_t* a, const int64_t* b, int64_t* r) {
     add_i64_kernel<<<(unsigned)((nd + 255) / 256), 256, 0, st>>>(a, b, r, nd);
@@ -748,37 +750,34 @@ bool block_witness_dev(lgs_ctx* c, const int64_t* x, unsigned n, unsigned d, uns
   // attention: fields 7 q_qkv, qkv, scores, x_max, exp, sum_exp, q_prob, q_ao_heads, q_ao, q_apr,
   // x_out, rem_qkv, rem_sc, rem_ao_heads, rem_apr
   const int64_t* dx = dv;
-  layer_norm(dx, 1, 0, derr + 8);
+  layer_norm(dx, 1, 0, derr + NLIN);
   linear(fld(6), d, w[2], 3, 3 * (size_t)d, fld(7), fld(18), fld(8), derr);
   head_scores_kernel<<<(unsigned)((hnn + 127) / 128), 128, 0, st>>>(
-      fld(8), heads, n, dh, score_scale, fld(9), fld(19), derr + 9);
+      fld(8), heads, n, dh, score_scale, fld(9), fld(19), derr + NLIN + 1);
   LGS_LAUNCH_CHECK();
   const int64_t* dexp = in(exp_lut, exp_len);
   softmax_witness_kernel<<<(unsigned)((hn + 127) / 128), 128, 0, st>>>(
       fld(9), heads, n, dexp, exp_len, offset, scale, fld(10), fld(11), fld(12), fld(13),
-      derr + 10);
+      derr + NLIN + 2);
   LGS_LAUNCH_CHECK();
   head_values_kernel<<<(unsigned)((nd + 127) / 128), 128, 0, st>>>(
-      fld(13), fld(8), heads, n, dh, scale, fld(14), fld(20), fld(15), derr + 11);
+      fld(13), fld(8), heads, n, dh, scale, fld(14), fld(20), fld(15), derr + NLIN + 3);
   LGS_LAUNCH_CHECK();
-  linear(fld(15), d, w[4], 4, d, fld(16), fld(21), tmp, derr + 2);
+  linear(fld(15), d, w[4], 4, d, fld(16), fld(21), tmp, derr + LW_FLAGS);
   add(dx, tmp, fld(17));
   // mlp: fields 29 q_fc, fc, act, q_fpr, x_out, rem_fc, rem_fpr
-  layer_norm(fld(17), 5, 22, derr + 12);
-  linear(fld(28), d, w[8], 7, hidden, fld(29), fld(34), fld(30), derr + 4);
+  layer_norm(fld(17), 5, 22, derr + NLIN + 4);
+  linear(fld(28), d, w[8], 7, hidden, fld(29), fld(34), fld(30), derr + 2 * LW_FLAGS);
   const int64_t* dgelu = in(gelu_lut, gelu_len);
   lut_gather_kernel<<<(unsigned)std::min<size_t>((nh + 255) / 256, 148 * 8), 256, 0, st>>>(
-      fld(30), nh, dgelu, gelu_len, offset, fld(31), derr + 13);
+      fld(30), nh, dgelu, gelu_len, offset, fld(31), derr + NLIN + 5);
   LGS_LAUNCH_CHECK();
-  linear(fld(31), hidden, w[10], 8, d, fld(32), fld(35), tmp, derr + 6);
+  linear(fld(31), hidden, w[10], 8, d, fld(32), fld(35), tmp, derr + 3 * LW_FLAGS);
   add(fld(17), tmp, fld(33));
   int err[NERR];
   LGS_CUDA(cudaMemcpyAsync(err, derr, sizeof(err), cudaMemcpyDeviceToHost, st));
   LGS_CUDA(cudaStreamSynchronize(st));
-  for (int i = 0; i < 8; i += 2)
-    if (err[i] >= 16)
-      throw DeviceTimeout("linear witness: a bounded device wait gave up (code " +
-                          std::to_string(err[i]) + ")");
+  for (int i = 0; i < NLIN; i += LW_FLAGS) throw_if_timed_out(err + i);
   for (int e : err)
     if (e) return false;
   d2h_staged(c, out, o, off[36] * 8, st);

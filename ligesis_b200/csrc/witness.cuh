@@ -9,13 +9,14 @@
 
 namespace lgs {
 
-// Marks *p, which may lie in host memory: a plain store, since an atomic of every thread with a bad
-// value would cross PCIe one by one (28 ms against 0.15 for 31 x 768 x 2304 out of range).  set_err
-// leaves a code that a bounded wait has written.
+// What goes wrong in a linear layer, a word for each kind, so that no store replaces another's: a
+// result outside the i64 range, an operand outside the tensor path's encodings, and the code of a
+// bounded wait that gave up (16 and above), which flag_failure writes.
+enum LwFlag { LW_RESULT, LW_OPERAND, LW_WAIT, LW_FLAGS };
+// Marks one of the first two, which may lie in host memory: a plain store, since an atomic of every
+// thread with a bad value would cross PCIe one by one (28 ms against 0.15 for 31 x 768 x 2304 out of
+// range).
 __device__ __forceinline__ void set_flag(int* p) { *(volatile int*)p = 1; }
-__device__ __forceinline__ void set_err(int* p) {
-  if (*(volatile int*)p == 0) *(volatile int*)p = 1;
-}
 
 // 128-bit accumulator as (hi:lo); a product of two i64 is added exactly.
 // (two's complement in two words, added modulo 2^128 like the reference's i128)

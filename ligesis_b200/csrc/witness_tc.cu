@@ -77,8 +77,9 @@ struct WtArgs {
   unsigned nsp[2];
   unsigned long long* acc;
   unsigned* count;
-  int* err;                 // 1: a result leaves the i64 range; >= 16: a bounded wait gave up
+  int* err;                 // a result leaves the i64 range
   int* range;               // an operand outside the limb encodings
+  int* wait;                // the code (16 and above) of a bounded wait that gave up
   long long budget;
   const uint8_t* xl;        // the X limb tiles of every (row tile, chunk), x_limbs_kernel
   const uint32_t* xsum;     // sum of x' per (row tile, chunk, row)
@@ -337,7 +338,7 @@ __device__ __forceinline__ uint64_t wt_produce(const WtArgs& a, WtCta& s) {
       if (lane == 0)
         ok = tc::mbar_wait(s.empty0 + 8 * st, ((t / WT_STAGES) - 1) & 1, s.fail, a.budget);
       if (!__shfl_sync(0xffffffffu, ok, 0)) {
-        if (lane == 0 && !*s.fail) tc::flag_failure(s.fail, a.err, 18);
+        if (lane == 0 && !*s.fail) tc::flag_failure(s.fail, a.wait, 18);
         break;
       }
     }
@@ -380,7 +381,7 @@ __device__ __forceinline__ uint64_t wt_produce(const WtArgs& a, WtCta& s) {
         ok = tc::mbar_wait(s.full0 + 8 * st, (t / WT_STAGES) & 1, s.fail, a.budget) &&
              tc::mbar_wait(s.xbar0 + 8 * st, (t / WT_STAGES) & 1, s.fail, a.budget);
       if (!__shfl_sync(0xffffffffu, ok, 0)) {
-        if (lane == 0 && !*s.fail) tc::flag_failure(s.fail, a.err, 16);
+        if (lane == 0 && !*s.fail) tc::flag_failure(s.fail, a.wait, 16);
         break;
       }
       if (lane == 0) {
@@ -587,10 +588,10 @@ __global__ void __launch_bounds__(WT_THREADS, 2) linear_witness_tc_kernel(const 
           : "r"((uint32_t)got)
           : "memory");
       if (!all) {
-        if (!s_fail) tc::flag_failure(&s_fail, a.err, 19);
+        if (!s_fail) tc::flag_failure(&s_fail, a.wait, 19);
       } else {
         if (!wt_epilogue(a, wu, tmem, sx, warp, 0, 1, lane, tid == 0, &s_last, 0))
-          set_err(a.err);
+          set_flag(a.err);
       }
     }
   }
@@ -599,10 +600,10 @@ __global__ void __launch_bounds__(WT_THREADS, 2) linear_witness_tc_kernel(const 
     // before its stage was refilled): wait for those before the CTA may exit
     for (unsigned g = x_issued > WT_STAGES ? x_issued - WT_STAGES : 0; g < x_issued; ++g)
       if (!tc::mbar_wait_drain(xbar0 + 8 * (g % WT_STAGES), (g / WT_STAGES) & 1))
-        atomicExch(a.err, 20);
+        atomicExch(a.wait, 20);
     // every MMA issued so far has completed once this arrives: wait before the TMEM is freed
     tc::mma_commit(drain);
-    if (!tc::mbar_wait_drain(drain, 0)) atomicExch(a.err, 17);
+    if (!tc::mbar_wait_drain(drain, 0)) atomicExch(a.wait, 17);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -764,7 +765,7 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
         uint8_t* stage = stages + s * stage_bytes;
         if (limi >= WT_STAGES &&
             !warp_wait(lim_empty(s), ((limi / WT_STAGES) - 1) & 1, &s_fail, a.budget)) {
-          if (lane == 0 && !s_fail) tc::flag_failure(&s_fail, a.err, 18);
+          if (lane == 0 && !s_fail) tc::flag_failure(&s_fail, a.wait, 18);
           ok = false;
           break;
         }
@@ -784,7 +785,7 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
         for (int b = 0; b < WP_BOXES; ++b, ++rawi) {
           const unsigned slot = rawi % nraw;
           if (!warp_wait(raw_full(slot), (rawi / nraw) & 1, &s_fail, a.budget)) {
-            if (lane == 0 && !s_fail) tc::flag_failure(&s_fail, a.err, 21);
+            if (lane == 0 && !s_fail) tc::flag_failure(&s_fail, a.wait, 21);
             ok = false;
             break;
           }
@@ -802,7 +803,7 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
     if (tid == 0) {
       // the newest X copy of each stage may still be in flight: wait for it before exiting
       for (unsigned g = x_issued > WT_STAGES ? x_issued - WT_STAGES : 0; g < x_issued; ++g)
-        if (!tc::mbar_wait_drain(xbar(g % WT_STAGES), (g / WT_STAGES) & 1)) atomicExch(a.err, 20);
+        if (!tc::mbar_wait_drain(xbar(g % WT_STAGES), (g / WT_STAGES) & 1)) atomicExch(a.wait, 20);
     }
   }
   else if (warp == WP_LOAD_WARP) {
@@ -818,7 +819,7 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
             const unsigned slot = rawi % nraw;
             if (rawi >= nraw &&
                 !tc::mbar_wait(raw_empty(slot), ((rawi / nraw) - 1) & 1, &s_fail, a.budget)) {
-              if (!s_fail) tc::flag_failure(&s_fail, a.err, 22);
+              if (!s_fail) tc::flag_failure(&s_fail, a.wait, 22);
               ok = false;
               break;
             }
@@ -835,7 +836,7 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
       }
       // the newest load of each slot may still be in flight: wait for it before exiting
       for (unsigned g = rawi > nraw ? rawi - nraw : 0; g < rawi; ++g)
-        if (!tc::mbar_wait_drain(raw_full(g % nraw), (g / nraw) & 1)) atomicExch(a.err, 24);
+        if (!tc::mbar_wait_drain(raw_full(g % nraw), (g / nraw) & 1)) atomicExch(a.wait, 24);
     }
   } else if (warp == WP_MMA_WARP) {
     // ---- MMA issue: unit i accumulates in set i % 2 once the epilogue has drained that set;
@@ -848,7 +849,7 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
         const WtUnit w = wt_unit(a, u);
         const unsigned b = i & 1;
         if (i >= 2 && !tc::mbar_wait(acc_empty(b), ((i / 2) - 1) & 1, &s_fail, a.budget)) {
-          if (!s_fail) tc::flag_failure(&s_fail, a.err, 23);
+          if (!s_fail) tc::flag_failure(&s_fail, a.wait, 23);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -857,7 +858,7 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
           const unsigned s = limi % WT_STAGES, ph = (limi / WT_STAGES) & 1;
           if (!tc::mbar_wait(lim_full(s), ph, &s_fail, a.budget) ||
               !tc::mbar_wait(xbar(s), ph, &s_fail, a.budget)) {
-            if (!s_fail) tc::flag_failure(&s_fail, a.err, 16);
+            if (!s_fail) tc::flag_failure(&s_fail, a.wait, 16);
             ok = false;
             break;
           }
@@ -883,7 +884,7 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
       }
       // every MMA issued so far has completed once this arrives: wait before the TMEM is freed
       tc::mma_commit(drain);
-      if (!tc::mbar_wait_drain(drain, 0)) atomicExch(a.err, 17);
+      if (!tc::mbar_wait_drain(drain, 0)) atomicExch(a.wait, 17);
     }
   } else {
     // ---- epilogue (warps 10-17: TMEM lane quarter warp % 4, row groups of half (warp - 10) / 4)
@@ -910,13 +911,13 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
           : "r"((uint32_t)got), "r"(128 * WP_EPI_HALVES)
           : "memory");
       if (!all) {
-        if (!s_fail) tc::flag_failure(&s_fail, a.err, 19);
+        if (!s_fail) tc::flag_failure(&s_fail, a.wait, 19);
         break;
       }
       const int64_t wpad = (int64_t)((size_t)w.nch * WT_KC - (w.ke - w.kb)) << 15;
       if (!wt_epilogue(a, w, tmem + b * WT_NG * nr, sx, q, h, WP_EPI_HALVES, lane, et == 0, &s_last,
                        wpad))
-        set_err(a.err);
+        set_flag(a.err);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(acc_empty(b));
@@ -936,7 +937,7 @@ __global__ void __launch_bounds__(WP_THREADS, 1)
 void linear_witness_tc(lgs_ctx* c, const int64_t* dx, size_t rows, size_t inner,
                        const int64_t* dw, size_t cols, bool w_transposed, const int64_t* db,
                        int64_t divisor, int64_t* dq, int64_t* dr, int64_t* dy, uint64_t* df,
-                       int* derr, int* drange) {
+                       int* flags) {
   cudaStream_t st = c->st;
   // row tiles of at most 63 x rows (plus the ones row), balanced
   const size_t ntr = (rows + WT_NR_MAX - 2) / (WT_NR_MAX - 1);
@@ -1009,8 +1010,9 @@ void linear_witness_tc(lgs_ctx* c, const int64_t* dx, size_t rows, size_t inner,
   }
   Arena& ar = c->arena;
   WtArgs a{dx, dw, db, rows, inner, cols, nr, nrv, w_transposed ? 1 : 0, divisor, dq, dr, dy, df};
-  a.err = derr;
-  a.range = drange;
+  a.err = flags + LW_RESULT;
+  a.range = flags + LW_OPERAND;
+  a.wait = flags + LW_WAIT;
   a.budget = c->wait_cycles
                  ? (long long)std::min<uint64_t>(c->wait_cycles, (uint64_t)tc::DRAIN_CYCLES)
                  : tc::DRAIN_CYCLES;
