@@ -155,9 +155,12 @@ WEIGHT_NAMES = ("ln_1_g", "ln_1_b", "attn_w", "attn_b", "attn_proj_w", "attn_pro
 
 def _block_on_device(x, w: dict, exp_lut, gelu_lut, cfg: dict, ctx: Context):
     """`block_witness` as one native call (lgs_block_witness), or None where the layers are run one
-    by one: arrays that are not the block's plain shapes, or values that call leaves to them."""
+    by one: arrays that are not the block's plain shapes, linear layers without a bias (None), or
+    values that call leaves to them."""
     n, d = cfg["n_seq"], cfg["d_model"]
     H = cfg.get("n_head", 12)
+    if any(w[k] is None for k in WEIGHT_NAMES):
+        return None
     host = lambda a: np.ascontiguousarray(a, dtype=np.int64)
     ws = [host(w[k]) for k in WEIGHT_NAMES]
     hid = ws[8].shape[-1]
@@ -196,8 +199,8 @@ def block_witness(x, w: dict, exp_lut, gelu_lut, cfg: dict = GPT2_31,
     """One block of the integer GPT-2 forward (model.rs:213-221): ln1, attention (qkv, per-head
     scores, softmax, weighted values, projection, residual), ln2 and the MLP (fc, GELU lookup,
     projection, residual), every step on the GPU.  `w` holds WEIGHT_NAMES (matrices row-major:
-    attn_w d x 3d, attn_proj_w d x d, fc_w d x hidden, fproj_w hidden x d).  Returns the witness
-    keyed by BLOCK_FIELDS."""
+    attn_w d x 3d, attn_proj_w d x d, fc_w d x hidden, fproj_w hidden x d; a linear layer's bias
+    may be None).  Returns the witness keyed by BLOCK_FIELDS."""
     n, d = cfg["n_seq"], cfg["d_model"]
     H = cfg.get("n_head", 12)
     dh = d // H
