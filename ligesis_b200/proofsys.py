@@ -185,9 +185,9 @@ def _block_on_device(x, w: dict, exp_lut, gelu_lut, cfg: dict, ctx: Context):
     p = lambda a: a.ctypes.data_as(i64p)
     done = C.c_int(0)
     check(load().lgs_block_witness(ctx.handle, p(x), n, d, H, hid, (i64p * 12)(*map(p, ws)),
-                                   p(luts[0]), luts[0].size, p(luts[1]), luts[1].size, sc,
-                                   sc * int(round(dh ** 0.5)), cfg["max_v"] * sc, p(out),
-                                   C.byref(done)))
+                                   p(luts[0]), luts[0].size, p(luts[1]), luts[1].size, int(sc),
+                                   int(sc * int(round(dh ** 0.5))), int(cfg["max_v"] * sc),
+                                   p(out), C.byref(done)))
     if not done.value:
         return None
     return {f: out[o:o + size].reshape(shape)

@@ -1,5 +1,5 @@
-"""A block whose linear layers have no bias runs layer by layer.  The CPU test looks at the route
-alone, the GPU test at the results."""
+"""The forms of a block's arguments: linear layers without a bias, which run layer by layer (the CPU
+test looks at the route alone), and scales that are not Python ints."""
 import numpy as np
 import pytest
 
@@ -26,5 +26,16 @@ def test_block_without_biases_matches_oracle(lgs, orc, names):
     zero = {k: np.zeros_like(v) if k in names else v for k, v in w.items()}
     want = orc.block_witness(x, zero, el, gl, CFG)
     got = ps.block_witness(x, _without(w, names), el, gl, CFG)
+    for k in ps.BLOCK_FIELDS:
+        assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("as_type", [float, np.int64, np.float64])
+def test_block_scale_of_any_number_type(lgs, orc, as_type):
+    x, w, el, gl = ps.synthetic_block(7, CFG)
+    want = orc.block_witness(x, w, el, gl, CFG)
+    cfg = {**CFG, "scale": as_type(CFG["scale"]), "max_v": as_type(CFG["max_v"])}
+    got = ps.block_witness(x, w, el, gl, cfg)
     for k in ps.BLOCK_FIELDS:
         assert np.array_equal(got[k], want[k]), k
