@@ -17,6 +17,9 @@
 // barrier each; a long one is bound by its products on the integer pipes.  Passes of two rounds
 // with a one-CTA end of ten sequential rounds took 38 us for that end and 473 us for three factors
 // of 2^22; tiles take 20 us and 406 us.
+// One or two factors have few products per entry, and a tile's high parts are runs of 2^(10 - r)
+// entries, which DRAM reads badly once the vector is longer than L2: sc_stream_kernel halves such
+// vectors twice per pass, in registers.
 //
 // Binary variant (the B_I check of pcs/src/ligesis.rs:423-428, factors [b, b - 1, eq]): the
 // middle factor is always the first minus one (folding is affine), so only b and eq are stored
@@ -30,8 +33,13 @@ namespace {
 constexpr unsigned SC_THREADS = 512;
 constexpr unsigned SC_LOG_T = 10;   // tile entries per factor
 constexpr unsigned SC_MAX_R = 8;    // rounds per pass: at least 64-byte runs of global memory
-constexpr unsigned SC_MAX_PASSES = 5;
-constexpr unsigned SC_MAX_K = 40;
+constexpr unsigned SC_MAX_K = 30;   // as the C ABI
+// Vectors of one or two factors are streamed from 2^23 entries on (134 MB a factor, against an L2
+// of 126 MB), two rounds per pass.  Device time with tiles alone and as it is: one factor 2^23 208
+// and 125 us, 2^24 377 and 218, 2^27 2663 and 1115; two factors 2^23 402 and 291, 2^24 748 and 535,
+// 2^27 5599 and 3431.  Three factors are bound by their products in tiles too (2^24: 1249 us).
+constexpr unsigned SC_STREAM_LOG = 23, SC_STREAM_R = 2, SC_STREAM_THREADS = 256;
+constexpr unsigned SC_MAX_PASSES = 6;  // 2^30: four streamed passes to 2^22, then two of tiles
 
 __device__ __forceinline__ ef2 shfl_xor_ef(ef2 v, int m) {
   ef2 r;
@@ -338,6 +346,71 @@ __global__ void __launch_bounds__(SC_THREADS, 2)
   }
 }
 
+// Rounds t0, .. of blockIdx.y's sumcheck on vectors of `len` entries: a thread owns the entries
+// i + m len / 2^R whose folds meet, holds them in registers, and keeps its sums there to the end.
+// What bounds it is its products again (first pass over two factors of 2^24: 345 us, ALU pipe 66 %
+// busy, DRAM 23 %).
+template <int D>
+__global__ void __launch_bounds__(SC_STREAM_THREADS, 2)
+    sc_stream_kernel(const ScJobs<D> jobs, size_t len, unsigned t0, size_t stride) {
+  constexpr int R = SC_STREAM_R;
+  __shared__ uint32_t acc[R][D + 1][6];
+  const ScOne<D> jb = my_job(jobs);
+  const unsigned tid = threadIdx.x, lane = tid & 31;
+  if (tid < sizeof(acc) / 4) (&acc[0][0][0])[tid] = 0;
+  ef2 run[R][D + 1];
+#pragma unroll
+  for (int l = 0; l < R; ++l)
+#pragma unroll
+    for (int q = 0; q <= D; ++q) run[l][q] = ef_zero();
+  const size_t step = len >> R;
+  for (size_t i = (size_t)blockIdx.x * SC_STREAM_THREADS + tid; i < step;
+       i += (size_t)gridDim.x * SC_STREAM_THREADS) {
+    ef2 x[D][1 << R];
+#pragma unroll
+    for (int j = 0; j < D; ++j)
+#pragma unroll
+      for (int m = 0; m < 1 << R; ++m) x[j][m] = ((const ef2*)jb.src[j])[i + m * step];
+#pragma unroll
+    for (int l = 0; l < R; ++l) {
+      const ef2 rt = jb.ch[t0 + l];
+      const int h = 1 << (R - 1 - l);
+#pragma unroll
+      for (int m = 0; m < h; ++m) {
+        ef2 v[D], df[D];
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+          v[j] = x[j][m], df[j] = ef_sub(x[j][m + h], v[j]);
+          x[j][m] = ef_add(v[j], ef_mul(rt, df[j]));
+        }
+#pragma unroll
+        for (int q = 0; q <= D; ++q) {
+          if (q != 1 || t0 + l == 0) {  // later rounds' g(1): from the claim chain
+            ef2 pr = v[0];
+#pragma unroll
+            for (int j = 1; j < D; ++j) pr = ef_mul(pr, v[j]);
+            run[l][q] = ef_add(run[l][q], pr);
+          }
+          if (q < D)
+#pragma unroll
+            for (int j = 0; j < D; ++j) v[j] = ef_add(v[j], df[j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < D; ++j) jb.dst[j][i] = x[j][0];
+  }
+  __syncthreads();  // acc is clear
+#pragma unroll
+  for (int l = 0; l < R; ++l)
+#pragma unroll
+    for (int q = 0; q <= D; ++q) warp_add(run[l][q], acc[l][q], lane);
+  __syncthreads();
+  if (tid < R * (D + 1))
+    jb.part[(size_t)(t0 + tid / (D + 1)) * stride + (size_t)blockIdx.x * (D + 1) +
+            tid % (D + 1)] = acc_value(&acc[0][0][0] + 6 * tid);
+}
+
 template <int D, bool BIN>
 void sumcheck_run(const ScJob* js, unsigned njobs, unsigned k, cudaStream_t st,
                   unsigned max_blocks) {
@@ -357,17 +430,31 @@ void sumcheck_run(const ScJob* js, unsigned njobs, unsigned k, cudaStream_t st,
   }
   auto kern = sc_tile_kernel<D, BIN>;
   static_assert(SC_THREADS == 1u << (SC_LOG_T - 1), "one pair of a tile per thread");
+  static_assert(SC_MAX_PASSES >= (SC_MAX_K - SC_STREAM_LOG + SC_STREAM_R) / SC_STREAM_R +
+                                     (SC_STREAM_LOG - 1 - SC_LOG_T + SC_MAX_R - 1) / SC_MAX_R &&
+                    SC_MAX_PASSES >= (SC_MAX_K - SC_LOG_T + SC_MAX_R - 1) / SC_MAX_R,
+                "every plan fits ScPasses");
   constexpr size_t smem = sizeof(TileSmem<D, BIN>), smem_end = smem + sizeof(ChainSmem<D>);
   LGS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_end));
   ScPasses prev{};
   int bf0 = js[0].bf0;
   unsigned t = 0;
-  while (k - t > SC_LOG_T) {  // passes of about equally many rounds, down to one tile
-    const unsigned left = k - t - SC_LOG_T, np = (left + SC_MAX_R - 1) / SC_MAX_R;
-    const unsigned r = (left + np - 1) / np;
+  while (k - t > SC_LOG_T) {
     const size_t len = (size_t)1 << (k - t);
-    const unsigned nb = (unsigned)std::min<size_t>(cap, len >> SC_LOG_T);
-    kern<<<dim3(nb, njobs), SC_THREADS, smem, st>>>(jobs, len, SC_LOG_T, r, t, bf0, 0, stride, prev);
+    unsigned r = 0, nb = 0;
+    if constexpr (D <= 2 && !BIN)
+      if (k - t >= SC_STREAM_LOG && !bf0) {
+        r = SC_STREAM_R;
+        nb = cap;  // far fewer than the vector's threads
+        sc_stream_kernel<D><<<dim3(nb, njobs), SC_STREAM_THREADS, 0, st>>>(jobs, len, t, stride);
+      }
+    if (!r) {  // passes of about equally many rounds, down to one tile
+      const unsigned left = k - t - SC_LOG_T, np = (left + SC_MAX_R - 1) / SC_MAX_R;
+      r = (left + np - 1) / np;
+      nb = (unsigned)std::min<size_t>(cap, len >> SC_LOG_T);
+      kern<<<dim3(nb, njobs), SC_THREADS, smem, st>>>(jobs, len, SC_LOG_T, r, t, bf0, 0, stride,
+                                                      prev);
+    }
     LGS_LAUNCH_CHECK();
     t += r;
     prev.t[prev.n] = t;
