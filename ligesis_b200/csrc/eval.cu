@@ -591,10 +591,11 @@ void rs_weights_dev(const ef2* r3, unsigned log2n, size_t n, const u64* tw, ef2*
 // ---- Basefold batched open ------------------------------------------------------------------
 // Level-0 combined codeword (pcs/src/basefold.rs:660-666, 735-741):
 // combined[i] = sum_ch coeffs[ch] sum_j eq4_ch[j] codes_ch[i][j].
-// Eight lanes share a row, reading it in 64-byte pieces; the products are summed as integers and
-// reduced once per lane.  A thread per row (strided reads, a reduction per product, the
+// 2^LG lanes share a row, reading it in pieces of as many values; the products are summed as
+// integers and reduced once per lane.  A thread per row (strided reads, a reduction per product, the
 // channels' eq tables one after another) left 2^11 rows on 8 SMs: 25 -> 9.5 us there, and 45 ->
 // 35 us for 2^17 rows of 64 base-field values.
+template <int LG>
 __global__ void __launch_bounds__(256)
     bf_combine_kernel(const BfChannelDev* __restrict__ chs, unsigned nch,
                       const ef2* __restrict__ coeffs, size_t D, ef2* __restrict__ combined) {
@@ -612,9 +613,10 @@ __global__ void __launch_bounds__(256)
     }
   }
   __syncthreads();
-  const unsigned l = threadIdx.x & 7;
-  for (size_t i0 = (size_t)blockIdx.x * 32; i0 < D; i0 += (size_t)gridDim.x * 32) {
-    const size_t i = i0 + (threadIdx.x >> 3);
+  constexpr unsigned LANES = 1u << LG, ROWS = 256 / LANES;
+  const unsigned l = threadIdx.x & (LANES - 1);
+  for (size_t i0 = (size_t)blockIdx.x * ROWS; i0 < D; i0 += (size_t)gridDim.x * ROWS) {
+    const size_t i = i0 + (threadIdx.x >> LG);
     Acc160 a0{}, a1{};
     if (i < D)
       for (unsigned c = 0; c < nch; ++c) {
@@ -623,7 +625,7 @@ __global__ void __launch_bounds__(256)
         if (chs[c].is_ef) {
           const ulonglong2* row = (const ulonglong2*)codes + i * L;
 #pragma unroll 4
-          for (unsigned j = l; j < L; j += 8) {
+          for (unsigned j = l; j < L; j += LANES) {
             const ulonglong2 x = __ldg(row + j);
             const ef2 w = wts[c][j];
             gl_mac(a0, w.c0, x.x);
@@ -634,7 +636,7 @@ __global__ void __launch_bounds__(256)
         } else {
           const u64* row = codes + i * L;
 #pragma unroll 8
-          for (unsigned j = l; j < L; j += 8) {
+          for (unsigned j = l; j < L; j += LANES) {
             const u64 x = __ldg(row + j);
             const ef2 w = wts[c][j];
             gl_mac(a0, w.c0, x);
@@ -644,15 +646,25 @@ __global__ void __launch_bounds__(256)
       }
     ef2 v = ef_make(gl_acc_reduce(a0), gl_acc_reduce(a1));
 #pragma unroll
-    for (int m = 4; m; m >>= 1) v = ef_add(v, shfl_xor_ef(v, m));
+    for (unsigned m = LANES / 2; m; m >>= 1) v = ef_add(v, shfl_xor_ef(v, m));
     if (i < D && l == 0) combined[i] = v;
   }
 }
-void bf_combine_dev(const BfChannelDev* chs_dev, unsigned nch, const ef2* coeffs, size_t D,
-                    ef2* combined, cudaStream_t st) {
+// li: the most columns a channel has, log2.  A lane takes eight values of such a row: with fewer its
+// two reductions cost more than its products (a whole Basefold prove, eight lanes a row and this
+// rule: 2^22 rows of one value 1060 -> 796 us, of four 629 -> 503 at 2^21, of eight 634 -> 534 at
+// 2^21, of 16 1026 -> 835 at 2^22, of 32 at 2^21 1327 -> 1025), with more 2^17 rows of 64 leave the
+// chip short of loads (286 us with eight lanes, 293 with two).
+void bf_combine_dev(const BfChannelDev* chs_dev, unsigned nch, unsigned li, const ef2* coeffs,
+                    size_t D, ef2* combined, cudaStream_t st) {
   if (nch > 4) throw ShapeError("basefold: at most 4 channels per launch");
-  const unsigned grid = std::min(cdiv(D, 32), 148u * 6);  // six CTAs of an SM fill it
-  bf_combine_kernel<<<grid, 256, 0, st>>>(chs_dev, nch, coeffs, D, combined);
+  const unsigned lg = li < 3 ? 0 : std::min(li - 3, 3u);
+  auto k = lg == 0   ? bf_combine_kernel<0>
+           : lg == 1 ? bf_combine_kernel<1>
+           : lg == 2 ? bf_combine_kernel<2>
+                     : bf_combine_kernel<3>;
+  const unsigned grid = std::min(cdiv(D, 256u >> lg), 148u * 6);  // six CTAs of an SM fill it
+  k<<<grid, 256, 0, st>>>(chs_dev, nch, coeffs, D, combined);
   LGS_LAUNCH_CHECK();
 }
 

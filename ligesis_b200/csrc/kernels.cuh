@@ -147,8 +147,8 @@ struct BfChannelDev {
   unsigned li;
   const ef2* point;  // num_vars = li + R coordinates
 };
-void bf_combine_dev(const BfChannelDev* chs_dev, unsigned nch, const ef2* coeffs, size_t D,
-                    ef2* combined, cudaStream_t st);
+void bf_combine_dev(const BfChannelDev* chs_dev, unsigned nch, unsigned li, const ef2* coeffs,
+                    size_t D, ef2* combined, cudaStream_t st);
 void bf_fold_poly_dev(const u64* const* pref, int is_ef, unsigned li, const ef2* point,
                       size_t out_len, ef2* m, cudaStream_t st);
 void bf_levels_dev(ef2* levels, size_t D, unsigned R, const ef2* ch, const u64* tw,

@@ -1154,7 +1154,8 @@ void prove_dev(lgs_ctx* c, const lgs_pk* pk, const lgs_commit_data* cd, const u6
   mark("main_suffix_start", st);
   // Stage B codeword chain on main (needs both prove-time commitments): combined level 0,
   // the R folds, and the Merkle trees of levels 1..R-1 (pcs/src/basefold.rs:735-784)
-  bf_combine_dev((const BfChannelDev*)(d_up + U_chs), 3, d_fields + fp.coeffs, D, levels, st);
+  bf_combine_dev((const BfChannelDev*)(d_up + U_chs), 3,
+                 *std::max_element(chan_li, chan_li + 3), d_fields + fp.coeffs, D, levels, st);
   bf_levels_dev(levels, D, R, d_fields + fp.ch_batch, c->tw.as<u64>(), st);
   mark("main_levels_end", st);
   if (R > 1) {
@@ -1421,7 +1422,7 @@ void basefold_prove_dev(lgs_ctx* c, const lgs_basefold* bf, const u64* point_hos
   // ---- device dataflow (pcs/src/basefold.rs:398-476) ----------------------------------------
   h2d(d_up, h_up, blob, st);
   eq_dot_dev(bf->poly.as<u64>(), B.is_ef ? 0 : 1, d_pt, n, (ef2*)(stage + S_y), part1, st);
-  bf_combine_dev((const BfChannelDev*)(d_up + U_chs), 1, (const ef2*)(d_up + U_one), L, levels,
+  bf_combine_dev((const BfChannelDev*)(d_up + U_chs), 1, li, (const ef2*)(d_up + U_one), L, levels,
                  st);
   bf_fold_poly_dev((const u64* const*)(d_up + U_ptr), B.is_ef, li, d_pt, mlen, mv, st);
   eq_dot_multi_dev((const EqDotTask*)(d_up + U_tasks), 2 * R, R, part2, st);
