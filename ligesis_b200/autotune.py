@@ -178,8 +178,11 @@ def tune_engine(lanes: int = 12, jobs: int = 96, repeats: int = 3, device: int =
     """Grid search of the engine lanes' launch choices on the batch workload (`jobs` polynomials
     of mu = floor(14 + 8u), host f in, proof out): with many small jobs in flight, smaller
     hash and sumcheck grids let kernels of different lanes share the SMs.  Keeps the setting
-    with the most proofs per second (best of `repeats` batches, host wall clock) and records it
-    per GPU name under "engine<lanes>"; every setting must give the same roots and proofs."""
+    with the most proofs per second and records it per GPU name under "engine<lanes>"; every
+    setting must give the same roots and proofs.  A batch's time is the engine's own, first
+    submission to last completion, the best of `repeats`: the copies of the proofs into Python
+    afterwards (30 MB a batch) take a third as long again when they land on fresh pages, and
+    whether they do depends on what the process holds, not on the setting."""
     import gc
 
     import ligesis_b200 as L
@@ -207,10 +210,9 @@ def tune_engine(lanes: int = 12, jobs: int = 96, repeats: int = 3, device: int =
                 def batch():
                     for o in oracles:
                         o.restart()
-                    res = eng.run([(pk, f, z, o) for (pk, f, z), o in zip(work, oracles)])
-                    return [(r.commit.root, r.proof.data) for r in res]
+                    return eng.run([(pk, f, z, o) for (pk, f, z), o in zip(work, oracles)])
 
-                out = batch()  # warm-up
+                out = [(r.commit.root, r.proof.data) for r in batch()]  # warm-up
                 if ref is None:
                     ref = out
                 if out != ref:
@@ -219,10 +221,9 @@ def tune_engine(lanes: int = 12, jobs: int = 96, repeats: int = 3, device: int =
                 for _ in range(repeats):
                     gc.collect()
                     gc.disable()
-                    t0 = time.perf_counter()
-                    batch()
-                    t = time.perf_counter() - t0
+                    res = batch()
                     gc.enable()
+                    t = (max(r.done_ms for r in res) - min(r.submit_ms for r in res)) / 1e3
                     t_best = t if t_best is None else min(t_best, t)
                 pps = round(len(work) / t_best, 1)
                 trials.append({"hash_ctas": h, "sumcheck_blocks": b, "pps": pps})
