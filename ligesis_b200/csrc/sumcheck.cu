@@ -10,7 +10,8 @@
 // sumcheck.  A tile is c consecutive low positions with all 2^r of their high parts (T = c 2^r
 // entries per factor): the pairs of r rounds lie inside it.  A CTA loads a tile, one pair per
 // thread, sums round 0 from registers and folds into shared memory, folds on, keeping every level,
-// and then sums the other rounds at once, again one pair per thread.  Persistent CTAs walk the tiles and leave one partial sum per round.
+// and then sums the other rounds at once, again one pair per thread.  Persistent CTAs walk the tiles
+// and leave one partial sum per round.
 // Vectors of at most 2^SC_LOG_T entries finish in one CTA, which also adds the earlier passes'
 // partials and fills in their g(1): g_t(1) = claim_t - g_t(0), claim_{t+1} = g_t(r_t), an affine
 // recurrence run as a scan.  What bounds a short vector is the chain of folds, one product and one
@@ -46,9 +47,6 @@ __device__ __forceinline__ ef2 shfl_xor_ef(ef2 v, int m) {
   r.c0 = __shfl_xor_sync(0xffffffffu, v.c0, m);
   r.c1 = __shfl_xor_sync(0xffffffffu, v.c1, m);
   return r;
-}
-__device__ __forceinline__ ef2 shfl_ef(ef2 v, unsigned src) {
-  return ef_make(__shfl_sync(0xffffffffu, v.c0, src), __shfl_sync(0xffffffffu, v.c1, src));
 }
 
 // Stored factor count: the binary variant keeps [b, eq] for the logical [b, b - 1, eq].
@@ -306,43 +304,38 @@ __global__ void __launch_bounds__(SC_THREADS, 2)
       for (int j = 0; j < S; ++j) jb.fin[j] = sm.sv[j][off];
     }
   }
-  if (warp != 0) return;
+  if (warp != 0 || t0 == 0) return;
   // The claim chain of the passes' rounds: with g_t(r) = sum_q L_q(r) g_t(q), claim_{t+1} = A_t +
   // L_1(r_t) claim_t, A_t collecting the other terms (and A_0 = g_0(r_0), whose g(1) is summed).
   // Lane t prepares round t's map and an inclusive scan of the compositions gives every lane
-  // claim_{t+1}; claim_t is the previous lane's, and the last lane's carries to the next 32 rounds.
-  ef2 carry = ef_zero();
-  for (unsigned b0 = 0; b0 < t0; b0 += 32) {
-    const unsigned t = b0 + lane, nt = min(32u, t0 - b0);
-    ef2 a = ef_zero(), w1 = ef_one(), g0 = ef_zero();
-    if (t < t0) {
-      g0 = cs.g[t][0];
-      w1 = t ? cs.w[t][1] : ef_zero();
-      a = ef_mul_ol(ef_sub(cs.w[t][0], w1), g0);
-      for (int q = t ? 2 : 1; q <= D; ++q) a = ef_add(a, ef_mul_ol(cs.w[t][q], cs.g[t][q]));
+  // claim_{t+1}; claim_t is the previous lane's.
+  static_assert(SC_MAX_K - SC_LOG_T <= 32, "a lane per round of the passes");
+  const unsigned t = lane;
+  ef2 a = ef_zero(), w1 = ef_one(), g0 = ef_zero();
+  if (t < t0) {
+    g0 = cs.g[t][0];
+    w1 = t ? cs.w[t][1] : ef_zero();
+    a = ef_mul_ol(ef_sub(cs.w[t][0], w1), g0);
+    for (int q = t ? 2 : 1; q <= D; ++q) a = ef_add(a, ef_mul_ol(cs.w[t][q], cs.g[t][q]));
+  }
+  for (unsigned off = 1; off < t0; off <<= 1) {
+    const ef2 pa = ef_make(__shfl_up_sync(0xffffffffu, a.c0, off),
+                           __shfl_up_sync(0xffffffffu, a.c1, off));
+    const ef2 pw = ef_make(__shfl_up_sync(0xffffffffu, w1.c0, off),
+                           __shfl_up_sync(0xffffffffu, w1.c1, off));
+    if (lane >= off) {
+      a = ef_add(a, ef_mul_ol(w1, pa));
+      w1 = ef_mul_ol(w1, pw);
     }
-    for (unsigned off = 1; off < nt; off <<= 1) {
-      const ef2 pa = ef_make(__shfl_up_sync(0xffffffffu, a.c0, off),
-                             __shfl_up_sync(0xffffffffu, a.c1, off));
-      const ef2 pw = ef_make(__shfl_up_sync(0xffffffffu, w1.c0, off),
-                             __shfl_up_sync(0xffffffffu, w1.c1, off));
-      if (lane >= off) {
-        a = ef_add(a, ef_mul_ol(w1, pa));
-        w1 = ef_mul_ol(w1, pw);
-      }
-    }
-    const ef2 incl = ef_add(a, ef_mul_ol(w1, carry));  // claim_{t + 1}
-    ef2 excl = ef_make(__shfl_up_sync(0xffffffffu, incl.c0, 1),
-                       __shfl_up_sync(0xffffffffu, incl.c1, 1));
-    if (lane == 0) excl = carry;  // claim_t
-    if (t < t0) {
-      ef2* out = jb.rounds + (size_t)t * (D + 1);
-      out[0] = g0;
-      out[1] = t ? ef_sub(excl, g0) : cs.g[0][1];
+  }
+  const ef2 claim = ef_make(__shfl_up_sync(0xffffffffu, a.c0, 1),
+                            __shfl_up_sync(0xffffffffu, a.c1, 1));  // claim_t, from t = 1 on
+  if (t < t0) {
+    ef2* out = jb.rounds + (size_t)t * (D + 1);
+    out[0] = g0;
+    out[1] = t ? ef_sub(claim, g0) : cs.g[0][1];
 #pragma unroll
-      for (int q = 2; q <= D; ++q) out[q] = cs.g[t][q];
-    }
-    carry = shfl_ef(incl, 31);
+    for (int q = 2; q <= D; ++q) out[q] = cs.g[t][q];
   }
 }
 
