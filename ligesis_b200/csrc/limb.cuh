@@ -61,21 +61,17 @@ __device__ __forceinline__ Limbs limb_rot(const Limbs& x) {
   return y;
 }
 // Natural-order radix-R DFTs (radix-2 DIT on bit-reversed inputs) of unpacked values, R = 2, 4, 8:
-// w_4 = 2^48; w_8 = 2^120, w_8^2 = 2^48, w_8^3 = 2^168.  ZH: the upper half of the inputs is zero
-// and not read.  The outputs' limbs are signed, at most 8 (2^24 - 1) in absolute value.
-template <int R, bool ZH>
+// w_4 = 2^48; w_8 = 2^120, w_8^2 = 2^48, w_8^3 = 2^168.  ZH (R = 8): the upper half of the inputs
+// is zero and not read.  The outputs' limbs are signed, at most 8 (2^24 - 1) in absolute value.
+template <int R, bool ZH = false>
 __device__ __forceinline__ void limb_dft(Limbs (&v)[R]) {
+  static_assert(R == 8 || !ZH, "only the first radix-8 of a padded row has zeros");
   if constexpr (R == 2) {
-    if constexpr (ZH) v[1] = v[0];
-    else limb_bfly<0>(v[0], v[1]);
+    limb_bfly<0>(v[0], v[1]);
   } else if constexpr (R == 4) {
     Limbs a0 = v[0], a1 = v[2], a2 = v[1], a3 = v[3];
-    if constexpr (ZH) {
-      a1 = a0, a3 = a2;
-    } else {
-      limb_bfly<0>(a0, a1);
-      limb_bfly<0>(a2, a3);
-    }
+    limb_bfly<0>(a0, a1);
+    limb_bfly<0>(a2, a3);
     limb_bfly<0>(a0, a2);
     limb_bfly<2>(a1, a3);
     v[0] = a0, v[1] = a1, v[2] = a2, v[3] = a3;
@@ -101,11 +97,11 @@ __device__ __forceinline__ void limb_dft(Limbs (&v)[R]) {
   }
 }
 // A DFT's output V = l0 + l1 2^24 + l2 2^48 + l3 2^72 mod p, some representative below 2^64: with
-// the offset the limbs are positive, below 2^28.2, and l1 >= 2^23.  2^72 = 2^40 - 2^8, so with u = l2 + (l3 >> 8) and the low byte of
-// l3 put at 2^40, V = l0 + (l1 - (l3 >> 16)) 2^24 - (l3 mod 2^16) 2^8 + Y 2^32, Y = u 2^16 + (l3
-// mod 2^8) 2^8 = y0 + y1 2^32, and Y 2^32 = y0 2^32 + y1 (2^32 - 1).  Everything but y0 2^32 sums
-// to a positive number below 2^54, so there is one carry out of 64 bits, and its 2^32 - 1 cannot
-// carry again.
+// the offset the limbs are positive, below 2^28.2, and l1 >= 2^23.  2^72 = 2^40 - 2^8, so with u =
+// l2 + (l3 >> 8) and the low byte of l3 put at 2^40, V = l0 + (l1 - (l3 >> 16)) 2^24 -
+// (l3 mod 2^16) 2^8 + Y 2^32, Y = u 2^16 + (l3 mod 2^8) 2^8 = y0 + y1 2^32, and Y 2^32 = y0 2^32 +
+// y1 (2^32 - 1).  Everything but y0 2^32 sums to a positive number below 2^54, so there is one
+// carry out of 64 bits, and its 2^32 - 1 cannot carry again.
 __device__ __forceinline__ u64 limb_pack(Limbs x) {
   limb_offset(x);
   const uint32_t l0 = x.l[0], l1 = x.l[1], l2 = x.l[2], l3 = x.l[3];
@@ -166,12 +162,12 @@ __device__ __forceinline__ u64 gl_mul_lazy(u64 x, u64 y) {
 #endif
 }
 // v <- its natural-order R-point DFT; any representatives in, some representatives out.
-template <int R, bool ZH = false>
+template <int R>
 __device__ __forceinline__ void dft_lazy(u64 (&v)[R]) {
   Limbs x[R];
 #pragma unroll
-  for (int i = 0; i < R; ++i) x[i] = limb_unpack(v[ZH ? i % (R / 2) : i]);
-  limb_dft<R, ZH>(x);
+  for (int i = 0; i < R; ++i) x[i] = limb_unpack(v[i]);
+  limb_dft<R>(x);
 #pragma unroll
   for (int i = 0; i < R; ++i) v[i] = limb_pack(x[i]);
 }

@@ -7,8 +7,9 @@
 // pass A  the 4096-point DFTs over k1 of 1, 2 or 4 consecutive columns k2 per CTA, as 64 x 64, each
 //         64-point DFT as radix-8 x radix-8 shared by 8 warps (one radix-8 per thread, a
 //         shared-memory exchange between the two), written as Z[k2][j1] (contiguous in j1).
-//         Global reads are 32-byte runs with 4 columns; the zeros of a padded row are never read.  N = 2^12 is finished here, and N = 2^13 too: a thread holds both columns of its
-//         row at the end and does the last radix-2.
+//         Global reads are 32-byte runs with 4 columns; the zeros of a padded row are never
+//         read.  N = 2^12 is finished here, and N = 2^13 too: a thread holds both columns of its row
+//         at the end and does the last radix-2.
 // pass B  the four-step twiddle w_N^(j1 k2) from a table laid out [k2][j1], then the N2-point
 //         DFT over k2; reads Z and writes X in 256-byte runs per warp.  N2 <= 32: one thread per
 //         column, in registers.  N2 = 64: 8 warps on 32 columns, an exchange between two radix-8.
@@ -175,9 +176,9 @@ __global__ void __launch_bounds__(256 * COLS, 4 / COLS)
 // loads Z[k2][j1] (256-byte rows), applies w_N^(j1 k2), does the radix-8 over kb, multiplies by
 // w_64^(jb ka), exchanges, and as jb = w does the radix-8 over ka: it then holds j' = w + 8 j0.
 // With R > 1 the outputs are multiplied by w_N2^(c j') and all but the last kept in the thread's
-// own slots of shared memory; a thread holds one j' for every c, so the radix-R over c needs no exchange.  The loop
-// over c is not unrolled: four copies of the eight warps' code missed the instruction cache
-// (2^20, 32 rows: 0.341 ms unrolled, 0.210 ms as it is).
+// own slots of shared memory; a thread holds one j' for every c, so the radix-R over c needs no
+// exchange.  The loop over c is not unrolled: four copies of the eight warps' code missed the
+// instruction cache (2^20, 32 rows: 0.341 ms unrolled, 0.210 ms as it is).
 constexpr size_t pb64_smem(int r) { return (size_t)(8 * 8 * 32 + (r - 1) * 8 * 256) * 8; }
 template <int R>
 __global__ void __launch_bounds__(256, R <= 2 ? 4 : 3)
@@ -253,7 +254,7 @@ __device__ __forceinline__ void pass_b_first(const u64* src, const u64* t4, u64 
       const size_t o = (size_t)(C + B * k) * 4096;
       y[k] = limb_unpack(C + B * k == 0 ? src[0] : gl_mul_lazy(src[o], __ldg(t4 + o)));
     }
-    limb_dft<A, false>(y);
+    limb_dft<A>(y);
     tw_pack<A, B, C, EL>(y, r);
     pass_b_first<A, B, EL, C + 1>(src, t4, r);
   }
