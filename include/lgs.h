@@ -280,8 +280,9 @@ lgs_status lgs_profile_get(lgs_ctx* ctx, const char* stage, double* total_ms, ui
 lgs_status lgs_profile_names(lgs_ctx* ctx, char* buf, size_t cap, size_t* needed);
 /* Launch choices of this context's kernels, picked by the autotuner (ligesis_b200/autotune.py;
  * no counterpart in the reference, which has no kernels).  0 restores the built-in default.
- *   "hash_ctas"        persistent CTAs of the subset-sum hash (default one per SM); fewer leave
- *                      SMs to the prove that runs beside the commit's hash
+ *   "hash_ctas"        persistent CTAs of the subset-sum hash (default one per SM), in pairs: an
+ *                      odd count is rounded down, and 1 gives two; fewer leave SMs to the prove
+ *                      that runs beside the commit's hash
  *   "sumcheck_blocks"  grid cap of the multi-CTA sumcheck passes (at most 296)
  *   "hash_groups"      commits of host polynomials: digest the codeword in this many row
  *                      groups (1..8) as their RS encoding finishes, under the upload

@@ -379,8 +379,8 @@ __global__ void __launch_bounds__(FS_THREADS, 3)
   }
 }
 
-// Shared memory of a tail: weight tables (2^FS_TAIL_LOG entries), the folded elements after the
-// first round (2^(FS_TAIL_LOG-1)), per-warp round sums (FS_TAIL_LOG x 16 warps x 3).
+// Shared memory of a tail: weight tables (2^FS_TAIL_LOG entries) and the folded elements after the
+// first round (2^(FS_TAIL_LOG-1)).
 constexpr size_t FS_TAIL_SMEM = ((size_t)1 << FS_TAIL_LOG) * sizeof(ef2) +
                                 ((size_t)1 << (FS_TAIL_LOG - 1)) * sizeof(Q4);
 constexpr unsigned FS_TAIL_THREADS = 512;  // latency-bound: as many warps as the registers allow

@@ -1,7 +1,11 @@
 // Shared-memory barriers, shared-memory matrix descriptors and the int8 tensor-core instructions
 // of sm_100a (tcgen05), as inline PTX, for the kernels that run on the 5th-generation tensor
-// cores (hash_tc.cu, witness_tc.cu).  Every wait is bounded: it gives up after a clock budget
-// (or when another role of the CTA has flagged a failure) instead of spinning for good.
+// cores (hash_tc.cu, witness_tc.cu).  Every wait on a barrier in shared memory is bounded: it
+// gives up after a clock budget (or when another role of the CTA has flagged a failure) instead of
+// spinning for good.  Two waits have no budget: a CTA pair's meetings (cluster_sync) and
+// tcgen05.alloc.  Both end: the halves of a pair are launched together and every wait before a
+// meeting is bounded; and an allocation waits only for CTAs that hold tensor memory on the same SM
+// and free it at their end (the hash's shared memory leaves room for no such CTA beside its own).
 #pragma once
 #include <cstdint>
 
@@ -123,9 +127,12 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
 }
-// Arrives on a barrier of either CTA of the pair (an address from map_to_rank).  The default CTA
-// scope: what it announces is shared memory or TMEM of the arriving CTA's own SM, which that SM's
-// tensor core reads, so no write has to travel; a cluster-scope release waits about 1000 clocks.
+// Arrives on a barrier of either CTA of the pair (an address from map_to_rank), with the default
+// CTA scope.  PTX orders only threads of one CTA by that, so that the leader's MMAs see what the
+// other CTA announces rests on how sm_100 runs them: it is shared memory or TMEM of the announcing
+// SM, which that SM's own tensor core reads, so no write has to travel.  Every digest of the tests
+// is compared with the oracle's.  A cluster-scope release, which PTX would ask for, waits about
+// 1000 clocks.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }

@@ -670,9 +670,9 @@ __global__ void add_i64_kernel(const int64_t* __restrict__ a, const int64_t* __r
 // staged, so the uploads (77 MB at GPT-2's sizes, most of the time) run under the layers before
 // them; nothing waits in between, and the results leave in one copy.  Layer by layer it was 34
 // calls, each uploading its inputs, waiting, and reading pageable results back (31 x 768, 12 heads,
-// hidden 3072: 13.9 -> 4.8 ms; the bytes alone take 1.5 ms of PCIe).  False, with
-// nothing written, when a value needs the layer-by-layer path: operands outside the tensor-core
-// encodings, or a range error that path reports.
+// hidden 3072: 13.3 -> 2.6 ms, of which PCIe takes 1.5 for the bytes alone).  False, with nothing
+// written, when a value needs the layer-by-layer path: operands outside the tensor-core encodings,
+// or a range error that path reports (9.2 ms with the attempt, 12.9 before).
 bool block_witness_dev(lgs_ctx* c, const int64_t* x, unsigned n, unsigned d, unsigned heads,
                        unsigned hidden, const int64_t* const w[12], const int64_t* exp_lut,
                        size_t exp_len, const int64_t* gelu_lut, size_t gelu_len, int64_t scale,
@@ -706,7 +706,8 @@ bool block_witness_dev(lgs_ctx* c, const int64_t* x, unsigned n, unsigned d, uns
   int* derr = ar.get<int>(NERR);
   LGS_CUDA(cudaMemsetAsync(derr, 0, NERR * sizeof(int), st));
   // Uploads go on a stream of their own, so that a ring slot is free as soon as its copy is done
-  // and not behind the layers enqueued before it (8.3 -> 4.8 ms per block).
+  // and not behind the layers enqueued before it (8.3 -> 4.8 ms per block when staging still went
+  // through the caches).
   cudaStream_t cp = c->side[0];
   LGS_CUDA(cudaEventRecord(c->ev_fork, st));  // the arena's earlier users are on the stream
   LGS_CUDA(cudaStreamWaitEvent(cp, c->ev_fork, 0));

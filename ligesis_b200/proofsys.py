@@ -200,7 +200,8 @@ def block_witness(x, w: dict, exp_lut, gelu_lut, cfg: dict = GPT2_31,
     scores, softmax, weighted values, projection, residual), ln2 and the MLP (fc, GELU lookup,
     projection, residual), every step on the GPU.  `w` holds WEIGHT_NAMES (matrices row-major:
     attn_w d x 3d, attn_proj_w d x d, fc_w d x hidden, fproj_w hidden x d; a linear layer's bias
-    may be None).  Returns the witness keyed by BLOCK_FIELDS."""
+    may be None).  Returns the witness keyed by BLOCK_FIELDS; its arrays may be views of one buffer,
+    so keeping one of them keeps them all (copy what is to outlive the rest)."""
     n, d = cfg["n_seq"], cfg["d_model"]
     H = cfg.get("n_head", 12)
     dh = d // H
