@@ -19,14 +19,19 @@ LIB = PKG / "liblgs.so"
 INCLUDE = PKG.parent / "include"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-# Host loops start on lines of their own: where the one that reduces an input's words fell decided
-# 12 % of a call on host arrays (lgs_subset_sum_hash, 128 x 4096: 1.15 or 1.30 ms), and any edit
-# elsewhere moves it.
 NVCC_FLAGS = ARCH + [
     "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
-    "-Xcompiler", "-falign-functions=64", "-Xcompiler", "-falign-loops=64",
     "--expt-relaxed-constexpr", "-Xcompiler", "-pthread", "-I", str(CSRC), "-I", str(INCLUDE),
 ]
+
+# Host code whose time depends on where the linker puts it, which any edit elsewhere moves: the loops
+# of the C entry points that reduce an input's words (12 % of lgs_subset_sum_hash on 128 x 4096, 1.15
+# or 1.30 ms) and the verifier's functions (2^7 x 2^17: 7.8 or 8.1 ms; its loops are better left as
+# they fall inside an aligned function).
+FILE_FLAGS = {
+    "capi.cu": ["-Xcompiler", "-falign-functions=64", "-Xcompiler", "-falign-loops=64"],
+    "verify.cpp": ["-Xcompiler", "-falign-functions=64"],
+}
 
 
 def _nvcc() -> str:
@@ -45,9 +50,10 @@ def _headers() -> list[Path]:
 
 
 def _compile(nvcc: str, src: Path, obj: Path, extra: list[str]) -> None:
-    cmd = [nvcc, *NVCC_FLAGS, *extra, "-c", str(src), "-o", str(obj)]
+    flags = [*NVCC_FLAGS, *FILE_FLAGS.get(src.name, []), *extra]
     if src.suffix == ".cpp":
-        cmd = [nvcc, *NVCC_FLAGS, *extra, "-x", "cu", "-c", str(src), "-o", str(obj)]
+        flags += ["-x", "cu"]
+    cmd = [nvcc, *flags, "-c", str(src), "-o", str(obj)]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"nvcc failed on {src.name}:\n{res.stdout}\n{res.stderr}")
