@@ -442,6 +442,7 @@ int verify_host(unsigned log_m, unsigned log_n, const Hash32& com_a, const Hash3
       EFv r4 = rev(ch);
       if (!sc_verify(pf.y4, pf.sc[2], o, &ch)) return false;
       EFv r5 = rev(ch);
+      if (r5.size() != log_w) return false;
       {  // v(r5) with v[i] = eq_{z1}[i/64] 2^(i%64): separable over the low 6 bits
         EFv lo(r5.begin(), r5.begin() + 6), hi(r5.begin() + 6, r5.end());
         EFv el = new_eq(lo), eh = new_eq(hi);
@@ -452,6 +453,7 @@ int verify_host(unsigned log_m, unsigned log_n, const Hash32& com_a, const Hash3
       }
       if (!sc_verify(pf.y4, pf.sc[3], o, &ch)) return false;
       EFv r3 = rev(ch);
+      if (r3.size() != log_n + 1) return false;
       {  // sel(r3) = sum_k eq_r2[k] eq_{r3}(idx[k]) (sel is zero elsewhere)
         ef2 sv = ef_zero();
         for (size_t k = 0; k < S; ++k) {
