@@ -65,8 +65,9 @@ lgs_status lgs_commit_device(lgs_ctx* ctx, const lgs_pk* pk, const uint64_t* f_d
                              uint8_t root[32], lgs_commit_data** out);
 /* Ligesis::commit without waiting for the device: the work is enqueued on the context's stream
  * and *out is at once usable by lgs_prove on the same context (stream order), so the prove's
- * host-side planning overlaps the commit's device work.  f is host memory (f_on_device = 0; read
- * before the call returns) or device memory of the context's device (f_on_device = 1; copied,
+ * host-side planning overlaps the commit's device work.  f is host memory (f_on_device = 0;
+ * pageable: read before the call returns; page-locked: read by the DMA engine, must stay allocated
+ * and unchanged until the commit is done) or device memory of the context's device (f_on_device = 1; copied,
  * must stay unchanged until the commit is done; f_on_device = 2: lent, not copied: the
  * commitment reads the caller's buffer until lgs_commit_data_free, so it must stay allocated
  * and unchanged until then, as the reference's commit owns f).  lgs_commit_root waits for the

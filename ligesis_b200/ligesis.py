@@ -213,6 +213,7 @@ class LigesisCommit:
         if self._root is None:
             r = np.zeros(32, dtype=np.uint8)
             check(load().lgs_commit_root(self._data.pk.ctx.handle, self._data.handle, ptr8(r)))
+            self._data.host_f = None  # the commit is done
             self._root, self._data = r.tobytes(), None
         return self._root
 
@@ -230,8 +231,9 @@ class CommitData:
     """Device-resident prover data retained between commit and prove (the reference keeps f,
     the bit columns, H and its Merkle tree, pcs/src/ligesis.rs:88-97)."""
 
-    def __init__(self, handle, pk: ProvingKey):
+    def __init__(self, handle, pk: ProvingKey, host_f: np.ndarray | None = None):
         self.handle, self.pk = handle, pk
+        self.host_f = host_f  # page-locked memory is still being read until the commit is done
 
     def codeword(self) -> np.ndarray:
         m, two_n = 1 << self.pk.log_m, 2 << self.pk.log_n
@@ -333,14 +335,16 @@ class Ligesis:
     @staticmethod
     def commit(pk: ProvingKey, f: MlPoly) -> tuple[LigesisCommit, CommitData]:
         """Enqueues the commit (lgs_commit_async) and returns at once: the root is read when
-        first used, and a prove on the same context runs after the commit on the device."""
+        first used, and a prove on the same context runs after the commit on the device.  Values in
+        page-locked memory must not change until then (they are kept alive); others have been read
+        when this returns."""
         if f.is_ext:
             raise ValueError("LigeSIS commits base-field polynomials")
         ev = f.evals
         h = vp()
         check(load().lgs_commit_async(pk.ctx.handle, pk.handle, ptr64(ev), ev.size, 0,
                                       C.byref(h)))
-        data = CommitData(h, pk)
+        data = CommitData(h, pk, ev)
         return LigesisCommit(data=data), data
 
     @staticmethod
@@ -365,6 +369,7 @@ class Ligesis:
         check(load().lgs_prove(pk.ctx.handle, pk.handle, data.handle, ptr64(zz), zz.shape[0],
                                ptr64(oracle.fields), oracle.fields.shape[0], ptr64(oracle.ints),
                                oracle.ints.shape[0], ptr64(cur), C.byref(p), C.byref(n)))
+        data.host_f = None  # the commit is done
         return LigesisProof(C.string_at(p, n.value))
 
     @staticmethod
