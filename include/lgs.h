@@ -130,7 +130,8 @@ lgs_status lgs_basefold_verify(const uint8_t root[32], const uint64_t* point, si
 
 /* ---- GKR fraction sum and GKR-LogUp lookup (logup/src/frac_sum.rs, logup/src/lookup.rs) ----
  * EF arrays hold 2 u64 per value (c0, c1), canonical.  With on_device = 1 the input pointers are
- * device pointers on the context's device (16-byte aligned) and are only read; otherwise host
+ * device pointers on the context's device (16-byte aligned), their values complete before the call
+ * (its stream waits for no other), and are only read; otherwise host
  * memory.  `cursor` is the RandomOracle's fields cursor (in/out); these provers draw no ints.
  * Proofs are owned by the context until its next prove.
  *

@@ -126,7 +126,8 @@ class FracSum:
     def prove(p, q, oracle: RandomOracle, ctx: Context | None = None):
         """frac_sum::prove: (FracSumProof, point (k, 2), p_in(point), q_in(point)).  p None: every
         numerator is one (the query side of a lookup).  p and q are EF arrays on the host or
-        CUDA tensors on the context's device."""
+        CUDA tensors on the context's device whose values are complete: the context's stream does
+        not wait for the stream that writes them."""
         ctx = ctx or Context.default()
         qp, n, on_dev, keep_q = _input(q, ctx)
         if p is None:
@@ -202,7 +203,8 @@ class Lookup:
 
     @staticmethod
     def prove_with_opening_points(a, t, e, oracle: RandomOracle, ctx: Context | None = None):
-        """(LookupProof, zq, zt).  a, t, e are EF arrays on the host, or CUDA tensors."""
+        """(LookupProof, zq, zt).  a, t, e are EF arrays on the host, or CUDA tensors whose values
+        are complete, as for FracSum.prove."""
         ctx = ctx or Context.default()
         ap, m, on_a, ka = _input(a, ctx)
         tp, n, on_t, kt = _input(t, ctx)
